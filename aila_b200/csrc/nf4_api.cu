@@ -515,13 +515,12 @@ AilaNf4Status run_decode(const AilaNf4Linear* l, AilaNf4Scratch* sc, const void*
 // ---------------------------------------------------------------------------------------
 namespace nf4 {
 
-AilaNf4Status ensure_mid_partials(AilaNf4Scratch* sc, size_t bytes) {
-    if (sc->mid_partials_bytes >= bytes) return AILA_NF4_OK;
-    if (sc->d_mid_partials) NF4_CUDA(cudaFree(sc->d_mid_partials));
-    sc->d_mid_partials = nullptr;
-    sc->mid_partials_bytes = 0;
-    NF4_CUDA(cudaMalloc(reinterpret_cast<void**>(&sc->d_mid_partials), bytes));
-    sc->mid_partials_bytes = bytes;
+// Partial tiles of the tensor-memory kernel's stream split, one size for every call (39 MB on 148 SMs):
+// captured launches keep the address, so the buffer neither grows nor moves until the scratch is destroyed.
+AilaNf4Status ensure_mid_partials(AilaNf4Scratch* sc) {
+    if (sc->d_mid_partials) return AILA_NF4_OK;
+    NF4_CUDA(cudaMalloc(reinterpret_cast<void**>(&sc->d_mid_partials),
+                        gemm_midrows_partial_bytes(sc->sm_count, kMidRowsMax)));
     return AILA_NF4_OK;
 }
 
@@ -812,12 +811,8 @@ AILA_NF4_API AilaNf4Status aila_nf4_scratch_reserve(AilaNf4Scratch* sc, int seq_
         // accumulation tiles of the small-batch kernel (16 rows x 32 batch columns of fp32 per row tile)
         st = ensure_rows_acc(sc, tiles * nf4::kTileRows * 32 * sizeof(float));
         if (st != AILA_NF4_OK) return st;
-        // partial tiles of the tensor-memory kernel: for small batches of any size, for the rows announced,
-        // and for every pass of a prompt where the GEMM route's buffer is asked for (calls that are captured
-        // allocate nothing)
-        const int rows = need_weight ? nf4::kMidRowsMax : seq_len < 64 ? 64 : seq_len;
-        st = nf4::ensure_mid_partials(
-            sc, nf4::gemm_midrows_partial_bytes(sc->sm_count, rows < nf4::kMidRowsMax ? rows : nf4::kMidRowsMax));
+        // partial tiles of the tensor-memory kernel (calls that are captured allocate nothing)
+        st = nf4::ensure_mid_partials(sc);
         if (st != AILA_NF4_OK) return st;
     }
     if (need_weight) {

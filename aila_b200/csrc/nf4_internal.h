@@ -50,8 +50,7 @@ struct AilaNf4Scratch {
     size_t partials_floats = 0;
     float* d_rows_acc = nullptr;  // accumulation tiles of the K-sliced small-batch kernel (kept zero)
     size_t rows_acc_bytes = 0;
-    float* d_mid_partials = nullptr;  // partial tiles of the tensor-memory kernel's stream split
-    size_t mid_partials_bytes = 0;
+    float* d_mid_partials = nullptr;  // partial tiles of the tensor-memory kernel's stream split (never moves)
     int* d_counters = nullptr;
     size_t counters_ints = 0;
     int* d_status = nullptr;  // device status word written by bounded waits
@@ -198,7 +197,7 @@ constexpr int kMidRowsMax = 256;
 bool gemm_midrows_supported(const AilaNf4Linear& w, int64_t swiglu_ff);
 int gemm_midrows_tiles(const AilaNf4Linear& w, int64_t swiglu_ff);  // counters it needs
 size_t gemm_midrows_partial_bytes(int ctas, int rows);  // of the stream split
-AilaNf4Status ensure_mid_partials(AilaNf4Scratch* sc, size_t bytes);
+AilaNf4Status ensure_mid_partials(AilaNf4Scratch* sc);
 AilaNf4Status launch_gemm_midrows(const AilaNf4Linear& w, AilaNf4Scratch& sc, const void* x, void* y,
                                   const void* residual, int rows, int64_t swiglu_ff, cudaStream_t s);
 

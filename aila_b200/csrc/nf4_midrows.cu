@@ -779,7 +779,7 @@ AilaNf4Status launch_gemm_midrows(const AilaNf4Linear& w, AilaNf4Scratch& sc, co
     const int64_t want = p.split > 0 ? (int64_t)p.n_tiles * p.split : (total + 7) / 8;  // stream: eight items per CTA at least
     const int grid = (int)(p.split > 0 || want < sc.sm_count ? want : sc.sm_count);
     if (p.split == 0) {
-        const AilaNf4Status st = ensure_mid_partials(&sc, gemm_midrows_partial_bytes(grid, rows));
+        const AilaNf4Status st = ensure_mid_partials(&sc);
         if (st != AILA_NF4_OK) return st;
         p.partials = sc.d_mid_partials;
     }

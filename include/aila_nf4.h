@@ -138,7 +138,7 @@ AILA_NF4_API void aila_nf4_scratch_destroy(AilaNf4Scratch* scratch);
  * CUDA graph). Mirrors Bnb4BitLinearScratch::ensure (src/ops/Bnb4BitLinear.cpp:414-451);
  * need_weight != 0 reserves the [out,in] bf16 weight buffer the seq_len > 1 route uses; seq_len > 1
  * also reserves the fp32 accumulation tiles of the small-batch decode kernel (128 bytes per output row)
- * and the partial tiles of the tensor-memory kernel (1 KB per SM and activation row, 64 to 256 rows).
+ * and the partial tiles of the tensor-memory kernel (256 KB per SM, allocated once and never moved).
  * A decode call for more than 262,144 output rows that was not reserved for grows the work space
  * inside the call: it allocates and waits for the device, so it cannot be captured.
  */

@@ -77,3 +77,41 @@ def test_gate_up(nf4, scratch, ff, k, m):
     assert ((out[:m].double() - want).abs() <= bound).all()
     assert (out[m] == 7.0).all()
     scratch.check()
+
+
+def test_captured_call_outlives_larger_calls(nf4):
+    """A captured call whose tiles span CTAs (152 tiles over the whole chip) keeps the address of the partial
+    tiles: calls with more rows on the same scratch must neither move nor free them. Every size of the row
+    range between the capture and the replay, then the same bits again."""
+    ff, k = 9728, 2560
+    g, u = _linear(nf4, 5, ff, k), _linear(nf4, 6, ff, k)
+    f = nf4.Bnb4BitLinear()
+    assert f.init_fused_rows(g, u), f.last_error
+    sc = nf4.Bnb4BitLinearScratch(0)
+    sc.ensure(64, k, 2 * ff, False)
+    x = _x(64, 64, k)
+    out = torch.empty(64, ff, dtype=torch.bfloat16, device="cuda")
+    call = nf4.Bnb4BitLinear.try_forward_decode_gate_up_swiglu
+    assert call(f, sc, x, out, ff, 64)
+    want = out.clone()
+    st = torch.cuda.Stream()
+    with torch.cuda.stream(st):
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=st):
+            assert call(f, sc, x, out, ff, 64)
+    larger = [(m, _x(m, m, k), torch.empty(m, ff, dtype=torch.bfloat16, device="cuda")) for m in (77, 200, 256, 384)]
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    for m, xm, om in larger:
+        assert call(f, sc, xm, om, ff, m)
+    torch.cuda.synchronize()
+    assert torch.cuda.mem_get_info()[0] == free, "the calls allocated or freed device memory"
+    # had the address been given back, an allocation of that size would now sit where the graph writes
+    guard = [torch.zeros(n * 2 ** 20 // 4, dtype=torch.int32, device="cuda") for n in (10, 12, 20, 31, 39)]
+    with torch.cuda.stream(st):
+        out.zero_()
+        graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, want)
+    assert all(int(t.count_nonzero()) == 0 for t in guard)
+    sc.check()
