@@ -324,7 +324,8 @@ AilaNf4Status ensure_weight(AilaNf4Scratch* sc, size_t bytes) {
     }
     NF4_CUDA(e);
     sc->weight_bytes = bytes;
-    return AILA_NF4_OK;
+    // whoever may run the GEMM route under capture may run the tensor-memory kernel with fewer rows
+    return nf4::ensure_mid_partials(sc);
 }
 
 using nf4::ensure_counters;
@@ -451,6 +452,13 @@ AilaNf4Status run_mid_rows(const AilaNf4Linear* l, AilaNf4Scratch* sc, const voi
                            int seq_len, int64_t ff_dim, cudaStream_t s) {
     AilaNf4Status st = ensure_counters(sc, (size_t)nf4::gemm_midrows_tiles(*l, ff_dim));
     if (st != AILA_NF4_OK) return st;
+    // The first call that is not captured allocates the partial tiles whatever split it takes itself: after
+    // it, calls of every split can be captured. (A captured first call fails only where its split needs them.)
+    if (!sc->d_mid_partials) {
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        NF4_CUDA(cudaStreamIsCapturing(s, &capture));
+        if (capture == cudaStreamCaptureStatusNone && (st = nf4::ensure_mid_partials(sc)) != AILA_NF4_OK) return st;
+    }
     const int passes = (seq_len + nf4::kMidRowsMax - 1) / nf4::kMidRowsMax;
     const size_t n_out = (size_t)(ff_dim > 0 ? ff_dim : l->N);
     for (int i = 0, m = 0; i < passes; ++i) {
@@ -808,7 +816,7 @@ AILA_NF4_API AilaNf4Status aila_nf4_scratch_reserve(AilaNf4Scratch* sc, int seq_
     AilaNf4Status st = ensure_counters(sc, tiles);
     if (st != AILA_NF4_OK) return st;
     if (seq_len > 1) {
-        // accumulation tiles of the small-batch kernel (16 rows x 32 batch columns of fp32 per row tile)
+        // accumulation tiles of the K-sliced kernel (16 rows x 32 batch columns of fp32 per row tile)
         st = ensure_rows_acc(sc, tiles * nf4::kTileRows * 32 * sizeof(float));
         if (st != AILA_NF4_OK) return st;
         // partial tiles of the tensor-memory kernel (calls that are captured allocate nothing)

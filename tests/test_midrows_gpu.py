@@ -115,3 +115,32 @@ def test_captured_call_outlives_larger_calls(nf4):
     assert torch.equal(out, want)
     assert all(int(t.count_nonzero()) == 0 for t in guard)
     sc.check()
+
+
+@pytest.mark.parametrize("before", ["weight buffer", "prompt", "other split"])
+def test_capture_after(nf4, before):
+    """What makes a call of 77 rows capturable: a reservation of the weight buffer alone, a longer prompt
+    through the dequantise + GEMM route, a call that took the other split and needed no partial tiles."""
+    n, k = 19456, 2560
+    lin = _linear(nf4, 9, n, k)
+    sc = nf4.Bnb4BitLinearScratch(0)
+    if before == "weight buffer":
+        sc.ensure(1, k, n, True)
+    elif before == "prompt":
+        lin.forward(sc, _x(1, 400, k), torch.empty(400, n, dtype=torch.bfloat16, device="cuda"), 400)
+    else:
+        small = _linear(nf4, 10, 2560, 4096)
+        small.forward(sc, _x(2, 77, 4096), torch.empty(77, 2560, dtype=torch.bfloat16, device="cuda"), 77)
+    x, y = _x(77, 77, k), torch.empty(77, n, dtype=torch.bfloat16, device="cuda")
+    torch.cuda.synchronize()
+    st = torch.cuda.Stream()
+    with torch.cuda.stream(st):
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=st):
+            lin.forward(sc, x, y, 77)
+        graph.replay()
+    torch.cuda.synchronize()
+    got = y.clone()
+    lin.forward(sc, x, y, 77)
+    assert torch.equal(got, y)
+    sc.check()
