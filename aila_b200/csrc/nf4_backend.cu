@@ -43,18 +43,18 @@ __device__ __forceinline__ float block_sum_128(float v, float* scratch) {
 // One block of 128 threads per query head and per key head; a key head's block also appends k and v to
 // the cache at position pos. The normalised row stays in shared memory until it is rotated. Latency-bound:
 // 4.8 us (cold L2) against 6.3 us with a nine-barrier reduction, the row through global memory and k behind
-// q in one block.
+// q in one block. The kernel is resident while the launch before still writes q, k, v and the position: they
+// are read from L2 (a non-coherent load of data that changes in the kernel's lifetime is undefined).
 __global__ void __launch_bounds__(128)
-prepare_qkv_kernel(uint16_t* __restrict__ q, uint16_t* __restrict__ k, const uint16_t* __restrict__ v,
-                   const float* __restrict__ rope_freq, const uint16_t* __restrict__ q_norm_w,
-                   const uint16_t* __restrict__ k_norm_w, uint16_t* __restrict__ k_cache,
-                   uint16_t* __restrict__ v_cache, int max_seq_len, int pos, const int* __restrict__ pos_dev,
-                   int n_q, int head_dim, float eps) {
+prepare_qkv_kernel(uint16_t* q, uint16_t* k, const uint16_t* v, const float* __restrict__ rope_freq,
+                   const uint16_t* __restrict__ q_norm_w, const uint16_t* __restrict__ k_norm_w,
+                   uint16_t* __restrict__ k_cache, uint16_t* __restrict__ v_cache, int max_seq_len, int pos,
+                   const int* pos_dev, int n_q, int head_dim, float eps) {
     __shared__ float scratch[128];
     extern __shared__ uint16_t normed[];  // [head_dim]
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");  // the launch before may still write q, k, v or the position
-    if (pos_dev) pos = *pos_dev;
+    if (pos_dev) pos = __ldcg(pos_dev);
     if (pos < 0 || pos >= max_seq_len) return;  // (the host refuses such a step; nothing is written)
     const bool is_q = (int)blockIdx.x < n_q;
     const int head = is_q ? blockIdx.x : blockIdx.x - n_q;
@@ -63,12 +63,12 @@ prepare_qkv_kernel(uint16_t* __restrict__ q, uint16_t* __restrict__ k, const uin
     const int half = head_dim / 2;
     float ss = 0.0f;
     for (int d = threadIdx.x; d < head_dim; d += 128) {
-        const float a = bf16_bits_to_f32(x[d]);
+        const float a = bf16_bits_to_f32(__ldcg(x + d));
         ss += a * a;
     }
     const float rms = sqrtf(block_sum_128(ss, scratch) / (float)head_dim + eps);
     for (int d = threadIdx.x; d < head_dim; d += 128)
-        normed[d] = f32_to_bf16_bits((bf16_bits_to_f32(x[d]) / rms) * bf16_bits_to_f32(w[d]));
+        normed[d] = f32_to_bf16_bits((bf16_bits_to_f32(__ldcg(x + d)) / rms) * bf16_bits_to_f32(w[d]));
     __syncthreads();
     const size_t at = ((size_t)head * max_seq_len + pos) * head_dim;
     for (int d = threadIdx.x; d < half; d += 128) {
@@ -84,7 +84,7 @@ prepare_qkv_kernel(uint16_t* __restrict__ q, uint16_t* __restrict__ k, const uin
         }
     }
     if (is_q) return;
-    for (int d = threadIdx.x; d < head_dim; d += 128) v_cache[at + d] = v[(size_t)head * head_dim + d];
+    for (int d = threadIdx.x; d < head_dim; d += 128) v_cache[at + d] = __ldcg(v + (size_t)head * head_dim + d);
 }
 
 // One block per query head: scores over the cached positions in shared memory, softmax, value sum.
@@ -176,9 +176,8 @@ __device__ __forceinline__ void cp_async_16(void* dst, const void* src) {
 
 template <int HD, int HG>
 __global__ void __launch_bounds__(kAttThreads)
-attention_cluster_kernel(const uint16_t* __restrict__ q, const uint16_t* __restrict__ k_cache,
-                         const uint16_t* __restrict__ v_cache, uint16_t* __restrict__ out, int heads_per_kv,
-                         int cached_len, const int* __restrict__ pos_dev, int max_seq_len) {
+attention_cluster_kernel(const uint16_t* q, const uint16_t* k_cache, const uint16_t* v_cache, uint16_t* out,
+                         int heads_per_kv, int cached_len, const int* pos_dev, int max_seq_len) {
     namespace cg = cooperative_groups;
     constexpr int TK = kAttKRows<HD>, KP = kAttKPitch<HD>;
     extern __shared__ __align__(16) uint8_t att_cl[];
@@ -190,7 +189,8 @@ attention_cluster_kernel(const uint16_t* __restrict__ q, const uint16_t* __restr
     float* s_score = reinterpret_cast<float*>(s_v + 2 * kAttVBytes);  // [HG][pitch]
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");  // the launch before writes q and the newest position
-    if (pos_dev) cached_len = min(*pos_dev + 1, cached_len);  // (the launch holds `cached_len` scores at most)
+    // (everything that the launch before may have written is read from L2: __ldcg, cp.async.cg)
+    if (pos_dev) cached_len = min(__ldcg(pos_dev) + 1, cached_len);  // (the launch holds `cached_len` scores at most)
     if (cached_len <= 0) return;                              // (the whole grid)
     cg::cluster_group cluster = cg::this_cluster();
     const int S = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
@@ -222,7 +222,7 @@ attention_cluster_kernel(const uint16_t* __restrict__ q, const uint16_t* __restr
     if (t_begin < t_end) load_k(t_begin);
     else asm volatile("cp.async.commit_group;" ::: "memory");
     load_v(0);
-    for (int i = tid; i < HG * HD; i += kAttThreads) s_q[i] = bf16_bits_to_f32(q[(size_t)head0 * HD + i]);
+    for (int i = tid; i < HG * HD; i += kAttThreads) s_q[i] = bf16_bits_to_f32(__ldcg(q + (size_t)head0 * HD + i));
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");  // every CTA of the cluster runs
 
     // ---- scores ----

@@ -190,7 +190,8 @@ __device__ __forceinline__ void emit(const MidParams& p, int tile, int quarter, 
         for (int k = 0; k < C; ++k) {
             if (m0 + k < p.M) {
                 const size_t at = (size_t)(m0 + k) * p.n_out + nn;
-                p.y[at] = f32_to_bf16_bits(p.residual ? v[k] + bf16_bits_to_f32(p.residual[at]) : v[k]);
+                // (from L2: the launch before may have written it while this one was resident)
+                p.y[at] = f32_to_bf16_bits(p.residual ? v[k] + bf16_bits_to_f32(__ldcg(p.residual + at)) : v[k]);
             }
         }
     }

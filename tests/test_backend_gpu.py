@@ -110,6 +110,59 @@ def test_attention_decode_cluster(be, heads, kv, hd, length):
     assert torch.allclose(out.cpu().double().view(heads, hd), want, rtol=2 ** -8, atol=1e-4)
 
 
+def test_step_replayed_with_new_inputs(be):
+    """q, k, v and the position are written by the launches right before and sit at the same addresses on
+    every replay; the kernels that read them start before those launches end. 200 replayed steps against the
+    same calls on fresh tensors with a wait after each."""
+    from aila_b200 import linear as nf4
+    heads, kv, hd, window, K = 8, 2, 64, 256, 512
+    qkv = nf4.Bnb4BitLinear()
+    assert qkv.init(make_weight(77, (heads + 2 * kv) * hd, K), 0), qkv.last_error
+    o = nf4.Bnb4BitLinear()
+    assert o.init(make_weight(78, K, heads * hd), 0), o.last_error
+    sc = nf4.Bnb4BitLinearScratch(0)
+    gen = torch.Generator().manual_seed(5)
+    w = torch.ones(hd, dtype=torch.bfloat16, device="cuda")
+    freq = (1e4 ** (-2 * torch.arange(hd // 2, dtype=torch.float64) / hd)).float().cuda()
+
+    def step(x, buf, att, y, kc, vc, pos, wait):
+        q, k, v = buf[0].split([heads * hd, kv * hd, kv * hd])
+        qkv.forward(sc, x, buf, 1)
+        wait()
+        be.decode_prepare_qkv(q, k, v, freq, w, w, kc, vc, 0, heads, kv, hd, 1e-6, pos)
+        wait()
+        be.attention_decode(q, kc, vc, att, heads, kv, hd, window, pos)
+        wait()
+        o.forward(sc, att.view(1, -1), y, 1)
+        wait()
+
+    def tensors():
+        z = lambda *s: torch.zeros(*s, dtype=torch.bfloat16, device="cuda")
+        return z(1, (heads + 2 * kv) * hd), z(heads * hd), z(1, K)
+    caches = [[torch.zeros(kv, window, hd, dtype=torch.bfloat16, device="cuda") for _ in range(2)] for _ in range(2)]
+    pos = torch.zeros(1, dtype=torch.int32, device="cuda")
+    x = torch.zeros(1, K, dtype=torch.bfloat16, device="cuda")
+    buf, att, y = tensors()
+    st = torch.cuda.Stream()
+    step(x, buf, att, y, *caches[0], pos, torch.cuda.synchronize)
+    with torch.cuda.stream(st):
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=st):
+            step(x, buf, att, y, *caches[0], pos, lambda: None)
+    inputs = _rand_bf16(gen, 200, 1, K).cuda()
+    torch.cuda.synchronize()
+    for t in range(200):
+        with torch.cuda.stream(st):
+            x.copy_(inputs[t])
+            pos.fill_(t)
+            graph.replay()
+        torch.cuda.synchronize()
+        fresh = tensors()
+        step(inputs[t].clone(), *fresh, *caches[1], pos.clone(), torch.cuda.synchronize)
+        assert all(torch.equal(a, b) for a, b in zip((buf, att, y, *caches[0]), (*fresh, *caches[1]))), t
+    sc.check()
+
+
 def test_backend_rejects_bad_arguments(be):
     from aila_b200 import _lib
     q = torch.zeros(1, 128, dtype=torch.bfloat16, device="cuda")

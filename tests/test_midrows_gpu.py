@@ -144,3 +144,38 @@ def test_capture_after(nf4, before):
     lin.forward(sc, x, y, 77)
     assert torch.equal(got, y)
     sc.check()
+
+
+@pytest.mark.parametrize("m", [16, 77])
+def test_residual_of_the_launch_before(nf4, m):
+    """The residual is what the launch before has just written, at the same address on every replay: it must
+    not come from a cache that an earlier replay filled."""
+    a, b = _linear(nf4, 41, 512, 512), _linear(nf4, 42, 512, 512)
+    sc = nf4.Bnb4BitLinearScratch(0)
+    sc.ensure(m, 512, 512, True)
+    x, y1, y2 = (torch.zeros(m, 512, dtype=torch.bfloat16, device="cuda") for _ in range(3))
+    st = torch.cuda.Stream()
+    with torch.cuda.stream(st):
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=st):
+            for _ in range(4):
+                a.forward(sc, x, y1, m)
+                b.forward(sc, y1, y2, m, y1)
+                a.forward(sc, y2, y1, m, y2)
+                b.forward(sc, y1, x, m, y1)
+    for rep in range(20):
+        start = _x(1000 + rep, m, 512)
+        t1, t2, t = torch.empty_like(start), torch.empty_like(start), start.clone()
+        torch.cuda.synchronize()
+        with torch.cuda.stream(st):
+            x.copy_(start)
+            graph.replay()
+        torch.cuda.synchronize()
+        for _ in range(4):
+            for lin, src, dst, res in ((a, t, t1, None), (b, t1, t2, t1), (a, t2, t1, t2), (b, t1, t, t1)):
+                dst.fill_(float("nan"))
+                torch.cuda.synchronize()
+                lin.forward(sc, src, dst, m, None if res is None else res.clone())
+                torch.cuda.synchronize()
+        assert torch.equal(t, x), rep
+    sc.check()
