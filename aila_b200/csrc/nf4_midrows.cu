@@ -394,6 +394,8 @@ gemm_midrows_kernel(const __grid_constant__ CUtensorMap map_x, const MidParams p
         __syncwarp();
     } else if (warp == 1) {
         if (elect_one()) {
+            // (x cannot arrive before the launch before has ended: its time does not count against the limit)
+            asm volatile("griddepcontrol.wait;" ::: "memory");
             int s = 0, seg = 0, ch = 0, kb = i0 % KB;
             uint32_t xph = 0;
             bool ok = true;
@@ -462,10 +464,18 @@ gemm_midrows_kernel(const __grid_constant__ CUtensorMap map_x, const MidParams p
         float4 e = e_next;
         int ch = 0;      // chunk
         int c_slot = 0;  // ring slot of the next item
+        bool waited = false;
+        // Before the first bounded wait, for the same reason; and the launch before may still read what the
+        // drain writes (y, scratch).
+        auto wait_for_launch_before = [&]() {
+            if (!waited) asm volatile("griddepcontrol.wait;" ::: "memory");
+            waited = true;
+        };
         // the warp's part of one chunk: block kb, or nothing (the chunk is short)
         auto chunk = [&](int kb, bool have) {
             const int set = ch & 1;
             if (ch >= kSets) {  // the set's previous operands have been used
+                wait_for_launch_before();
                 ok = wait_spin(&done[set], ((ch >> 1) - 1) & 1, p.limit, abort_flag);
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) {
@@ -526,7 +536,6 @@ gemm_midrows_kernel(const __grid_constant__ CUtensorMap map_x, const MidParams p
         const int chunks = (p.M + 7) >> 3;    // accumulator columns in use, in eights
         const int row = quarter * 32 + lane;  // lane of the accumulator
         int seg = 0;
-        bool waited = false;
         uint32_t joins = 0;
         for (int ls = 0; ls < n && ok; ++seg) {
             const int tile = (i0 + ls) / KB;
@@ -538,6 +547,7 @@ gemm_midrows_kernel(const __grid_constant__ CUtensorMap map_x, const MidParams p
             if (!ok) break;
             // ---- drain the accumulator ----
             const int b = seg % bufs;
+            wait_for_launch_before();
             ok = wait_spin(&acc_full[b], (seg / bufs) & 1, p.limit, abort_flag);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) {
@@ -545,11 +555,6 @@ gemm_midrows_kernel(const __grid_constant__ CUtensorMap map_x, const MidParams p
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            if (!waited) {
-                // the previous launch may still read what is written from here on (y, scratch)
-                asm volatile("griddepcontrol.wait;" ::: "memory");
-                waited = true;
-            }
             const uint32_t dcol = tmem + lane_off + (uint32_t)(b * 128);
             const bool whole = kb0 == 0 && le - ls == KB;
             const size_t part = (size_t)kTileM * p.NB;
@@ -623,7 +628,7 @@ gemm_midrows_kernel(const __grid_constant__ CUtensorMap map_x, const MidParams p
             }
             ls = le;
         }
-        if (!waited) asm volatile("griddepcontrol.wait;" ::: "memory");
+        wait_for_launch_before();
         asm volatile("cp.async.wait_all;" ::: "memory");
         __syncwarp();
     }

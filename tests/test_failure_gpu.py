@@ -98,6 +98,42 @@ def test_chained_kernel_gives_up_and_recovers(nf4, oracle):
         o.close()
 
 
+def test_launch_before_does_not_count_against_the_limit(nf4):
+    """A few-row call right behind attention over a long context on one key/value head: its CTAs start on the
+    idle SMs and stay there until the attention has ended, far longer than the limit for their own waits."""
+    from aila_b200 import backend
+    w = make_weight(401, 2560, 4096)
+    l = _lin(nf4, w)
+    sc = nf4.Bnb4BitLinearScratch(0)
+    x = synth.gaussian_activation(12, 32, 4096).cuda()
+    y, want = (torch.empty(32, 2560, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    l.forward(sc, x, want, 32)
+    length = 25000
+    q = torch.randn(64, device="cuda").to(torch.bfloat16)
+    cache = torch.randn(1, length, 64, device="cuda").to(torch.bfloat16)
+    out = torch.empty_like(q)
+    backend.attention_decode(q, cache, cache, out, 1, 1, 64, length)
+    torch.cuda.synchronize()
+    t0, t1, t2 = (torch.cuda.Event(enable_timing=True) for _ in range(3))
+    t0.record()
+    backend.attention_decode(q, cache, cache, out, 1, 1, 64, length)
+    t1.record()
+    l.forward(sc, x, want, 32)
+    t2.record()
+    torch.cuda.synchronize()
+    attention_us, own_us = 1e3 * t0.elapsed_time(t1), 1e3 * t1.elapsed_time(t2)
+    assert attention_us > 4 * own_us, (attention_us, own_us)   # (what the test rests on)
+    sc.set_wait_limit(int(attention_us / 2 * MS / 1000))
+    for _ in range(3):
+        backend.attention_decode(q, cache, cache, out, 1, 1, 64, length)
+        l.forward(sc, x, y, 32)
+    torch.cuda.synchronize()
+    sc.check()
+    assert torch.equal(y, want)
+    l.close()
+    sc.close()
+
+
 def test_static_entry_reports_its_status(nf4):
     """The allocation-free entry point has a status word of its own; aila_nf4_static_check reads
     and clears it."""
