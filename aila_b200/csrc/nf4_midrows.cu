@@ -133,15 +133,25 @@ __device__ __forceinline__ void tmem_ld8(uint32_t addr, float (&v)[8]) {
     for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-// Bounded wait without back-off: the chain decode -> MMA -> free slot is latency-critical.
+// Bounded wait without back-off: the chain decode -> MMA -> free slot is latency-critical. The limit counts
+// from the end of the launch before, which this kernel is resident beside (x cannot arrive earlier): a wait
+// that runs out waits for that launch once and starts its clock again.
 __device__ __forceinline__ bool wait_spin(uint64_t* bar, uint32_t parity, long long limit, volatile int* abort_flag) {
     if (mbar_try_wait(bar, parity)) return true;
-    const long long t0 = clock64();
+    long long t0 = clock64();
+    bool alone = false;
+    const int tries = limit < 100000 ? 4 : 256;  // between two looks at the clock: a fraction of the limit
     while (true) {
 #pragma unroll 1
-        for (int i = 0; i < 256; ++i)
+        for (int i = 0; i < tries; ++i)
             if (mbar_try_wait(bar, parity)) return true;
-        if (*abort_flag || clock64() - t0 > limit) return false;
+        if (*abort_flag) return false;
+        if (clock64() - t0 > limit) {
+            if (alone) return false;
+            asm volatile("griddepcontrol.wait;" ::: "memory");
+            alone = true;
+            t0 = clock64();
+        }
     }
 }
 
@@ -184,14 +194,14 @@ __device__ __forceinline__ void emit(const MidParams& p, int tile, int quarter, 
                 p.y[(size_t)m * p.n_out + nn] = f32_to_bf16_bits(__fdividef(g, 1.0f + __expf(-g)) * u);
         }
     } else {
+        // (the residual by a plain load: the launch before is visible behind griddepcontrol.wait, to coherent loads)
         const int nn = tile * kTileM + quarter * 32 + lane;
         if (nn >= p.n_out) return;
 #pragma unroll
         for (int k = 0; k < C; ++k) {
             if (m0 + k < p.M) {
                 const size_t at = (size_t)(m0 + k) * p.n_out + nn;
-                // (from L2: the launch before may have written it while this one was resident)
-                p.y[at] = f32_to_bf16_bits(p.residual ? v[k] + bf16_bits_to_f32(__ldcg(p.residual + at)) : v[k]);
+                p.y[at] = f32_to_bf16_bits(p.residual ? v[k] + bf16_bits_to_f32(p.residual[at]) : v[k]);
             }
         }
     }
@@ -394,8 +404,6 @@ gemm_midrows_kernel(const __grid_constant__ CUtensorMap map_x, const MidParams p
         __syncwarp();
     } else if (warp == 1) {
         if (elect_one()) {
-            // (x cannot arrive before the launch before has ended: its time does not count against the limit)
-            asm volatile("griddepcontrol.wait;" ::: "memory");
             int s = 0, seg = 0, ch = 0, kb = i0 % KB;
             uint32_t xph = 0;
             bool ok = true;
@@ -464,18 +472,10 @@ gemm_midrows_kernel(const __grid_constant__ CUtensorMap map_x, const MidParams p
         float4 e = e_next;
         int ch = 0;      // chunk
         int c_slot = 0;  // ring slot of the next item
-        bool waited = false;
-        // Before the first bounded wait, for the same reason; and the launch before may still read what the
-        // drain writes (y, scratch).
-        auto wait_for_launch_before = [&]() {
-            if (!waited) asm volatile("griddepcontrol.wait;" ::: "memory");
-            waited = true;
-        };
         // the warp's part of one chunk: block kb, or nothing (the chunk is short)
         auto chunk = [&](int kb, bool have) {
             const int set = ch & 1;
             if (ch >= kSets) {  // the set's previous operands have been used
-                wait_for_launch_before();
                 ok = wait_spin(&done[set], ((ch >> 1) - 1) & 1, p.limit, abort_flag);
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) {
@@ -536,6 +536,7 @@ gemm_midrows_kernel(const __grid_constant__ CUtensorMap map_x, const MidParams p
         const int chunks = (p.M + 7) >> 3;    // accumulator columns in use, in eights
         const int row = quarter * 32 + lane;  // lane of the accumulator
         int seg = 0;
+        bool waited = false;
         uint32_t joins = 0;
         for (int ls = 0; ls < n && ok; ++seg) {
             const int tile = (i0 + ls) / KB;
@@ -547,7 +548,6 @@ gemm_midrows_kernel(const __grid_constant__ CUtensorMap map_x, const MidParams p
             if (!ok) break;
             // ---- drain the accumulator ----
             const int b = seg % bufs;
-            wait_for_launch_before();
             ok = wait_spin(&acc_full[b], (seg / bufs) & 1, p.limit, abort_flag);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) {
@@ -555,6 +555,11 @@ gemm_midrows_kernel(const __grid_constant__ CUtensorMap map_x, const MidParams p
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (!waited) {
+                // the previous launch may still read what is written from here on (y, scratch)
+                asm volatile("griddepcontrol.wait;" ::: "memory");
+                waited = true;
+            }
             const uint32_t dcol = tmem + lane_off + (uint32_t)(b * 128);
             const bool whole = kb0 == 0 && le - ls == KB;
             const size_t part = (size_t)kTileM * p.NB;
@@ -628,7 +633,7 @@ gemm_midrows_kernel(const __grid_constant__ CUtensorMap map_x, const MidParams p
             }
             ls = le;
         }
-        wait_for_launch_before();
+        if (!waited) asm volatile("griddepcontrol.wait;" ::: "memory");
         asm volatile("cp.async.wait_all;" ::: "memory");
         __syncwarp();
     }

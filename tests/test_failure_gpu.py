@@ -134,6 +134,36 @@ def test_launch_before_does_not_count_against_the_limit(nf4):
     sc.close()
 
 
+def test_few_row_kernel_gives_up_and_recovers(nf4):
+    """The tensor-memory kernel with waits of a single cycle, in both splits (clusters for 20 row tiles, the
+    chip-wide split for 152) and for one and several blocks of rows: the launch ends and reports the timeout;
+    with the default limit the same scratch then gives the right sums (the counters of tiles that CTAs share
+    are zero again)."""
+    sc = nf4.Bnb4BitLinearScratch(0)
+    for n, k in ((2560, 9728), (19456, 2560)):
+        l = _lin(nf4, make_weight(501, n, k))
+        w = l.dequantize_weight().double()
+        for m in (16, 77, 256):
+            x = synth.gaussian_activation(13, m, k).cuda()
+            y = torch.empty(m, n, dtype=torch.bfloat16, device="cuda")
+            sc.set_wait_limit(1)
+            for _ in range(3):
+                l.forward(sc, x, y, m)
+            torch.cuda.synchronize()
+            with pytest.raises(_lib.Nf4Error) as err:
+                sc.check()
+            assert err.value.status == _lib.ERR_KERNEL_TIMEOUT
+            sc.set_wait_limit(2_000_000_000)
+            for _ in range(2):
+                y.fill_(float("nan"))
+                l.forward(sc, x, y, m)
+                sc.check()
+                want = x.double() @ w
+                assert float((y.double() - want).norm() / want.norm()) < 5e-3
+        l.close()
+    sc.close()
+
+
 def test_static_entry_reports_its_status(nf4):
     """The allocation-free entry point has a status word of its own; aila_nf4_static_check reads
     and clears it."""
