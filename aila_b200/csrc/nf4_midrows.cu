@@ -568,6 +568,7 @@ gemm_midrows_kernel(const __grid_constant__ CUtensorMap map_x, const MidParams p
                     float v[8];
                     tmem_ld8(dcol + (uint32_t)(ch * 8), v);
                     emit(p, tile, quarter, lane, ch * 8, v);
+                    __syncwarp();  // (lanes past the output left early; the next load is warp-wide)
                 }
             } else {
                 // partial tile, to shared memory (every copy, look-up and MMA of this CTA is through with
@@ -629,6 +630,7 @@ gemm_midrows_kernel(const __grid_constant__ CUtensorMap map_x, const MidParams p
                         }
                         emit(p, tile, quarter, lane, ch * 8, v);
                     }
+                    __syncwarp();  // (lanes past the output left early; the next tile's loads are warp-wide)
                 }
             }
             ls = le;
