@@ -63,13 +63,16 @@ constexpr int kSets = 2;                 // operand sets of kGroups slots in ten
 constexpr int kSlotCols = kUnitK / 2;    // 64 bf16 per lane = 32 columns
 constexpr int kSlotCol0 = 256;           // accumulators below, operand slots from here
 constexpr int kMaxX = kSets * kGroups;   // blocks of x in the ring at most
-constexpr uint32_t kLut = 65536u;        // window offset of the look-up table (64 KB)
-constexpr uint32_t kXRing = 131072u;     // x ring
+constexpr uint32_t kLutBytes = 65536u;   // look-up table, at the first shared address that is a multiple of 64 KB
+constexpr uint32_t kXRing = 131072u;     // the x ring behind it starts here at the latest, counted from the CTA's first byte
+constexpr uint32_t kPart = 65536u;       // a cluster's partial tiles, at the same place in every CTA
 constexpr int kSmem = 227 * 1024;
 constexpr int kHeadBytes = 2048;         // barriers, code books
 constexpr int kDepth = 3;                // items a decode warp has in flight
 constexpr int kSlotBytes = 2 * kUnitStrideF32;  // one warp's part of an item: two units at most
-static_assert(2048 + kHeadBytes + kDecodeWarps * kDepth * kSlotBytes <= 65536, "weight ring below the table");
+constexpr uint32_t kRingEnd = kHeadBytes + kDecodeWarps * kDepth * kSlotBytes;
+static_assert(2048 + kRingEnd <= 65536, "weight ring below the table");
+static_assert(kPart + kTileM * 256 * 4 <= kSmem, "a partial tile of 256 columns");
 
 struct MidParams {
     const uint8_t* units;
@@ -212,10 +215,11 @@ gemm_midrows_kernel(const __grid_constant__ CUtensorMap map_x, const MidParams p
     extern __shared__ __align__(1024) uint8_t mid_smem[];
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const uint32_t base = smem_u32(mid_smem);
-    // In a cluster the CTA's shared addresses carry its rank above bit 24: places are offsets in the
-    // CTA's own window.
-    const uint32_t win = base & 0xff000000u;
-    uint8_t* const window = mid_smem - (base - win);  // generic address of window offset 0
+    // The table's lines are found by inserting a byte into an address, so it starts at a multiple of 64 KB of
+    // the address itself, whatever the upper bits of a CTA's shared addresses are in a cluster; everything
+    // else is counted from the CTA's first byte.
+    const uint32_t lut = (base + 0xffffu) & ~0xffffu;
+    const uint32_t lut_off = lut - base;
     uint64_t* x_full = reinterpret_cast<uint64_t*>(mid_smem);
     uint64_t* x_empty = x_full + kMaxX;
     uint64_t* a_full = x_empty + kMaxX;     // [kSets]
@@ -235,9 +239,9 @@ gemm_midrows_kernel(const __grid_constant__ CUtensorMap map_x, const MidParams p
     const float q_lane = __ldg(p.qmap + (lane & 15));
     const float n_mine = p.kind == kAbsmaxCodes && tid < 256 ? __ldg(p.nmap + tid) : 0.0f;
     const uint32_t x_bytes = (uint32_t)p.NB * 128u;
-    auto x_stage = [&](int s) { return kXRing + (uint32_t)s * x_bytes; };
-    // the table needs its fixed place in the shared window (the same for every CTA of every launch)
-    if (base - win > 2048u || base - win + kSmem < kXRing + (uint32_t)p.x_stages * x_bytes) {
+    auto x_stage = [&](int s) { return lut_off + kLutBytes + (uint32_t)s * x_bytes; };
+    // (the dynamic shared memory starts at most 2 KB behind a multiple of 64 KB)
+    if (lut_off < kRingEnd || lut_off + kLutBytes + (uint32_t)p.x_stages * x_bytes > kSmem) {
         if (tid == 0) atomicExch(p.status, kStatusBadArgument);
         if (p.split > 1) {  // (the rest of the cluster may look at this CTA's memory)
             cooperative_groups::this_cluster().sync();
@@ -350,7 +354,7 @@ gemm_midrows_kernel(const __grid_constant__ CUtensorMap map_x, const MidParams p
     for (int i = tid; i < 256 * 16; i += kThreads) {  // (whole warps)
         const int e = i >> 4;
         const float hi = __shfl_sync(0xffffffffu, q_lane, e >> 4), lo = __shfl_sync(0xffffffffu, q_lane, e & 15);
-        *reinterpret_cast<float4*>(window + kLut + (uint32_t)i * 16u) = make_float4(hi, lo, hi, lo);
+        *reinterpret_cast<float4*>(mid_smem + lut_off + (uint32_t)i * 16u) = make_float4(hi, lo, hi, lo);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -375,7 +379,7 @@ gemm_midrows_kernel(const __grid_constant__ CUtensorMap map_x, const MidParams p
                     if (i >= p.x_stages) ok = wait_spin(&x_empty[s], ph, p.limit, abort_flag);
                     if (!ok) break;
                     mbar_expect_tx(&x_full[s], x_bytes);
-                    tma_load_2d(window + x_stage(s), &map_x, kb * kUnitK, 0, &x_full[s]);
+                    tma_load_2d(mid_smem + x_stage(s), &map_x, kb * kUnitK, 0, &x_full[s]);
                     if (++kb == KB) kb = 0;
                     if (++s == p.x_stages) {
                         s = 0;
@@ -393,7 +397,7 @@ gemm_midrows_kernel(const __grid_constant__ CUtensorMap map_x, const MidParams p
                     if (!ok) break;
                     mbar_expect_tx(&x_full[set], (uint32_t)size * x_bytes);
                     for (int k = 0; k < size; ++k)
-                        tma_load_2d(window + x_stage(set * kGroups + k), &map_x, (kb + k) * kUnitK, 0, &x_full[set]);
+                        tma_load_2d(mid_smem + x_stage(set * kGroups + k), &map_x, (kb + k) * kUnitK, 0, &x_full[set]);
                     left -= size;
                     kb = kb + size == KB ? 0 : kb + size;
                 }
@@ -435,7 +439,7 @@ gemm_midrows_kernel(const __grid_constant__ CUtensorMap map_x, const MidParams p
                             const int st = p.x_per_item ? s : set * kGroups + k;
                             if (p.x_per_item) ok = wait_spin(&x_full[s], xph, p.limit, abort_flag);
                             if (ok) {
-                                const uint64_t bd = x_desc(x_stage(st));
+                                const uint64_t bd = x_desc(base + x_stage(st));
                                 const uint32_t a = tmem + kSlotCol0 + (uint32_t)((set * kGroups + k) * kSlotCols);
 #pragma unroll
                                 for (int j = 0; j < 4; ++j) {
@@ -466,7 +470,7 @@ gemm_midrows_kernel(const __grid_constant__ CUtensorMap map_x, const MidParams p
         }
         __syncwarp();
     } else if (warp >= kFirstDecodeWarp) {
-        const uint32_t lut_lane = win + kLut + (uint32_t)lane * 8u;
+        const uint32_t lut_lane = lut + (uint32_t)lane * 8u;
         const uint32_t lane_off = (uint32_t)(quarter * 32) << 16;
         bool ok = true;
         float4 e = e_next;
@@ -573,7 +577,7 @@ gemm_midrows_kernel(const __grid_constant__ CUtensorMap map_x, const MidParams p
             } else {
                 // partial tile, to shared memory (every copy, look-up and MMA of this CTA is through with
                 // it) or to the scratch
-                float4* o = p.split > 1 ? reinterpret_cast<float4*>(window + kLut)
+                float4* o = p.split > 1 ? reinterpret_cast<float4*>(mid_smem + kPart)
                                         : reinterpret_cast<float4*>(p.partials + ((size_t)c * 2 + (kb0 == 0 ? 1 : 0)) * part);
                 for (int ch = grp; ch < chunks; ch += kGroups) {
                     float v[8];
@@ -651,7 +655,7 @@ gemm_midrows_kernel(const __grid_constant__ CUtensorMap map_x, const MidParams p
         const int fours = warp >= kFirstDecodeWarp && !*abort_flag ? (p.M + 3) >> 2 : 0;
         bool arrived = false;
         for (int c4 = rank * kGroups + grp; c4 < fours; c4 += S * kGroups) {
-            float4* mine = reinterpret_cast<float4*>(window + kLut) + (size_t)c4 * kTileM + row;
+            float4* mine = reinterpret_cast<float4*>(mid_smem + kPart) + (size_t)c4 * kTileM + row;
             float4 a[8];
 #pragma unroll
             for (int s = 0; s < 8; ++s) a[s] = s < S ? *cluster.map_shared_rank(mine, s) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
