@@ -41,17 +41,20 @@ __device__ __forceinline__ float block_sum_128(float v, float* scratch) {
 }
 
 // One block of 128 threads per query head and per key head; a key head's block also appends k and v to
-// the cache at position pos. The normalised row stays in shared memory until it is rotated. Latency-bound:
+// the cache at position pos. The normalised row stays in shared memory until it is rotated (a row too long
+// for what every launch may use stays where it is). Latency-bound:
 // 4.8 us (cold L2) against 6.3 us with a nine-barrier reduction, the row through global memory and k behind
 // q in one block. The kernel is resident while the launch before still writes q, k, v and the position: they
 // are read from L2 (a non-coherent load of data that changes in the kernel's lifetime is undefined).
+constexpr int kPrepareShared = 20480;  // values of a row that fit beside the 512 static bytes in 48 KB
+
 __global__ void __launch_bounds__(128)
 prepare_qkv_kernel(uint16_t* q, uint16_t* k, const uint16_t* v, const float* __restrict__ rope_freq,
                    const uint16_t* __restrict__ q_norm_w, const uint16_t* __restrict__ k_norm_w,
                    uint16_t* __restrict__ k_cache, uint16_t* __restrict__ v_cache, int max_seq_len, int pos,
                    const int* pos_dev, int n_q, int head_dim, float eps) {
     __shared__ float scratch[128];
-    extern __shared__ uint16_t normed[];  // [head_dim]
+    extern __shared__ uint16_t prepare_row[];  // [head_dim] up to kPrepareShared
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");  // the launch before may still write q, k, v or the position
     if (pos_dev) pos = __ldcg(pos_dev);
@@ -59,6 +62,7 @@ prepare_qkv_kernel(uint16_t* q, uint16_t* k, const uint16_t* v, const float* __r
     const bool is_q = (int)blockIdx.x < n_q;
     const int head = is_q ? blockIdx.x : blockIdx.x - n_q;
     uint16_t* x = (is_q ? q : k) + (size_t)head * head_dim;
+    uint16_t* normed = head_dim <= kPrepareShared ? prepare_row : x;
     const uint16_t* w = is_q ? q_norm_w : k_norm_w;
     const int half = head_dim / 2;
     float ss = 0.0f;
@@ -433,12 +437,10 @@ AILA_NF4_API AilaNf4Status aila_decode_prepare_qkv(void* q_bf16, void* k_bf16, c
                                                        ", max_seq_len=" + std::to_string(max_seq_len) + ")");
     nf4::BackendDevGuard guard(device);
     if (guard.err != cudaSuccess) return nf4::cuda_fail(guard.err, "cudaSetDevice");
-    if (head_dim > 20480)  // (beyond the 48 KB a launch may use without asking)
-        NF4_CUDA(cudaFuncSetAttribute(nf4::prepare_qkv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, head_dim * 2));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(num_heads_q + num_kv_heads));
     cfg.blockDim = dim3(128);
-    cfg.dynamicSmemBytes = (size_t)head_dim * 2;
+    cfg.dynamicSmemBytes = head_dim <= nf4::kPrepareShared ? (size_t)head_dim * 2 : 0;
     cfg.stream = static_cast<cudaStream_t>(stream);
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;

@@ -67,6 +67,12 @@ def test_decode_prepare_qkv(be, heads, kv, hd, pos):
     assert not bf16_bits(kc)[:, pos + 1:].any() and not bf16_bits(kc)[:, :pos].any()
 
 
+@pytest.mark.parametrize("hd", [20478, 20480, 20482, 40000, 120000])
+def test_decode_prepare_qkv_long_heads(be, hd):
+    """Both sides of the row that fits in the shared memory of every launch, and a row that fits nowhere."""
+    test_decode_prepare_qkv(be, 2, 1, hd, 3)
+
+
 @pytest.mark.parametrize("heads,kv,hd,length", [(4, 2, 64, 1), (32, 8, 128, 300), (16, 16, 128, 2047), (8, 1, 256, 33)])
 def test_attention_decode(be, heads, kv, hd, length):
     gen = torch.Generator().manual_seed(200 + heads + length)
