@@ -547,6 +547,14 @@ AilaNf4Status ensure_counters(AilaNf4Scratch* sc, size_t tiles) {
     return AILA_NF4_OK;
 }
 
+bool overlapped_launches() {
+    static const bool on = [] {
+        const char* e = std::getenv("AILA_NF4_PDL");
+        return !(e && e[0] == '0');
+    }();
+    return on;
+}
+
 AilaNf4Status fail(AilaNf4Status code, const std::string& message) {
     g_last_error = message;
     return code;

@@ -446,7 +446,7 @@ AILA_NF4_API AilaNf4Status aila_decode_prepare_qkv(void* q_bf16, void* k_bf16, c
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = nf4::overlapped_launches() ? 1 : 0;
     NF4_CUDA(cudaLaunchKernelEx(&cfg, nf4::prepare_qkv_kernel, static_cast<uint16_t*>(q_bf16),
                                 static_cast<uint16_t*>(k_bf16), static_cast<const uint16_t*>(v_bf16), rope_freq,
                                 static_cast<const uint16_t*>(q_norm_weight_bf16),
@@ -494,7 +494,7 @@ AILA_NF4_API AilaNf4Status aila_attention_decode(const void* q_bf16, const void*
         attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[1].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
-        cfg.numAttrs = 2;
+        cfg.numAttrs = nf4::overlapped_launches() ? 2 : 1;
         NF4_CUDA(cudaLaunchKernelEx(&cfg, plan.fn, static_cast<const uint16_t*>(q_bf16),
                                     static_cast<const uint16_t*>(k_cache_bf16),
                                     static_cast<const uint16_t*>(v_cache_bf16), static_cast<uint16_t*>(out_bf16),

@@ -741,7 +741,7 @@ AilaNf4Status launch_gemm_common(const void* w_nk, const FusedWeight* fw, const 
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = overlapped_launches() ? 1 : 0;
     const FusedWeight none = {};
     cudaError_t e = fw ? cudaLaunchKernelEx(&cfg, gemm_bf16_tcgen05_kernel<true>, map_x, map_w, p, *fw)
                        : cudaLaunchKernelEx(&cfg, gemm_bf16_tcgen05_kernel<false>, map_x, map_w, p, none);

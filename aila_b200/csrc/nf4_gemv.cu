@@ -1257,10 +1257,6 @@ cudaError_t launch_stream_t(const StreamParams& p, int grid, int smem, cudaStrea
     // Programmatic dependent launch: the next kernel on the stream may start its set-up (table
     // build, first weight copies) while this one drains; it waits for our completion before it
     // reads x. Disabled with AILA_NF4_PDL=0.
-    static const bool use_pdl = [] {
-        const char* e = std::getenv("AILA_NF4_PDL");
-        return !(e && e[0] == '0');
-    }();
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
     cfg.blockDim = dim3(kStreamThreads);
@@ -1270,7 +1266,7 @@ cudaError_t launch_stream_t(const StreamParams& p, int grid, int smem, cudaStrea
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = use_pdl ? 1 : 0;
+    cfg.numAttrs = overlapped_launches() ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, gemv_stream_kernel<KIND, PAIRED, BATCH>, p);
 }
 
@@ -1720,10 +1716,6 @@ cudaError_t launch_rows_t(const RowsParams& p, int grid, cudaStream_t s) {
     }
     // Programmatic dependent launch, as for the streaming kernel: table build, barrier set-up and the
     // first weight copies overlap the previous kernel's tail. Disabled with AILA_NF4_PDL=0.
-    static const bool use_pdl = [] {
-        const char* e = std::getenv("AILA_NF4_PDL");
-        return !(e && e[0] == '0');
-    }();
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
     cfg.blockDim = dim3(kRowsThreads);
@@ -1733,7 +1725,7 @@ cudaError_t launch_rows_t(const RowsParams& p, int grid, cudaStream_t s) {
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = use_pdl ? 1 : 0;
+    cfg.numAttrs = overlapped_launches() ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, gemv_rows_kernel<KIND, RB>, p);
 }
 

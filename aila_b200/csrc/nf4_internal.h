@@ -80,6 +80,7 @@ namespace nf4 {
 // error plumbing (nf4_api.cu)
 AilaNf4Status fail(AilaNf4Status code, const std::string& message);
 AilaNf4Status cuda_fail(cudaError_t e, const char* what);
+bool overlapped_launches();  // programmatic dependent launch, of every kernel that uses it (AILA_NF4_PDL=0: none)
 #define NF4_CUDA(call)                                         \
     do {                                                       \
         cudaError_t e__ = (call);                              \

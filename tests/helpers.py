@@ -47,3 +47,32 @@ def concat_rows(ws):
     """Row concatenation of quantised weights with fp32 absmax, as init_fused_rows does
     (Bnb4BitLinear.cpp:604-615). Returns (packed, absmax_f32_list_placeholder)."""
     return np.concatenate([np.asarray(w.packed, np.uint8).reshape(-1) for w in ws])
+
+
+def captured(call, stream=None):
+    """Captures call() in a CUDA graph: (mangled names of the kernels it launches, how many of them may start
+    before the launch before has ended)."""
+    from cuda.bindings import driver
+    torch.cuda.synchronize()
+    stream = stream or torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        graph = torch.cuda.CUDAGraph(keep_graph=True)
+        with torch.cuda.graph(graph, stream=stream):
+            call()
+    torch.cuda.synchronize()
+
+    def ask(fn, *args):
+        err, *rest = fn(*args)
+        assert int(err) == 0, (fn.__name__, err)
+        return rest
+    raw = driver.CUgraph(graph.raw_cuda_graph())
+    nodes, count = ask(driver.cuGraphGetNodes, raw, 1024)
+    names = []
+    for node in nodes[:count]:
+        if ask(driver.cuGraphNodeGetType, node)[0] == driver.CUgraphNodeType.CU_GRAPH_NODE_TYPE_KERNEL:
+            params = ask(driver.cuGraphKernelNodeGetParams, node)[0]
+            name = ask(driver.cuKernelGetName, params.kern) if int(params.kern) else ask(driver.cuFuncGetName, params.func)
+            names.append(name[0].decode())
+    edges, count = ask(driver.cuGraphGetEdges_v2, raw, 1024)[2:]
+    programmatic = int(driver.CUgraphDependencyType.CU_GRAPH_DEPENDENCY_TYPE_PROGRAMMATIC)
+    return names, sum(int(e.type) == programmatic for e in edges[:count])
