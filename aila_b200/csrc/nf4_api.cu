@@ -354,32 +354,54 @@ AilaNf4Status ensure_io(void** buf, size_t* have, size_t need) {
     return AILA_NF4_OK;
 }
 
+// Integer value of an environment variable, or `unset`.
+int env_int(const char* name, int unset) {
+    const char* e = std::getenv(name);
+    return e && *e ? std::atoi(e) : unset;
+}
+
 // What the tensor-memory kernel (use_mid_rows below) does not take:
-// Small batches (2 .. AILA_NF4_DECODE_ROWS_MAX rows, default 48; 0 or 1 turns it off): batched decode
-// launches of up to 32 rows each (one pass over the weights per launch) instead of the dequantise +
+// Small batches (2 .. AILA_NF4_DECODE_ROWS_MAX rows, 48 when it is not set; 0 or 1 turns it off): batched
+// decode launches of up to 32 rows each (one pass over the weights per launch) instead of the dequantise +
 // GEMM route, when a small-batch kernel takes the shape and no bf16 weight cache exists (with a
 // cache the GEMM has nothing to dequantise). A pass of 32 and one of 16 rows still beat the GEMM
 // route (measured on the cfg4 stack: 5.0 ms against 5.6 ms per step at 48 rows; two passes of 32
 // rows, 5.9 ms, do not).
+constexpr int kDecodeRowsDefault = 48;
 int decode_rows_max() {
     static const int v = [] {
-        const char* e = std::getenv("AILA_NF4_DECODE_ROWS_MAX");
-        if (!e || !*e) return 48;
-        const int n = std::atoi(e);
+        const int n = env_int("AILA_NF4_DECODE_ROWS_MAX", kDecodeRowsDefault);
         return n < 0 ? 0 : (n > 128 ? 128 : n);
     }();
     return v;
 }
 
-// The K-sliced kernel (x slice of all rows in shared memory) serves 9 .. 32 rows where it takes the
-// linear and a decode kernel was asked for (the tensor-memory kernel comes first otherwise): up to eight rows the streaming kernel's batched form is faster (its x fragments from L2
-// cost less than the K-sliced kernel's accumulation in global memory).
-// AILA_NF4_ROWS_KERNEL=0 turns it off, =1 uses it from two rows on.
-bool use_rows_kernel(const AilaNf4Linear* l, int64_t ff_pair, int rows) {
-    static const int mode = [] {
-        const char* e = std::getenv("AILA_NF4_ROWS_KERNEL");
-        return (e && e[0] == '0') ? 0 : ((e && e[0] == '1') ? 1 : 2);
+// AILA_NF4_ROWS_KERNEL: 0 sends small batches to the streaming kernel's batched form only, 1 to the K-sliced
+// kernel from two rows on; anything else is as if it were not set (2).
+int rows_kernel_mode() {
+    static const int v = [] {
+        const int n = env_int("AILA_NF4_ROWS_KERNEL", 2);
+        return n == 0 || n == 1 ? n : 2;
     }();
+    return v;
+}
+
+// AILA_NF4_FUSED_PREFILL: 1 takes the GEMM that rebuilds its weight tiles from NF4 for prompts, 0 the
+// dequantisation pass and the GEMM, both also where the tensor-memory kernel would serve; otherwise -1.
+int fused_prefill_mode() {
+    static const int v = [] {
+        const int n = env_int("AILA_NF4_FUSED_PREFILL", -1);
+        return n == 0 || n == 1 ? n : -1;
+    }();
+    return v;
+}
+
+// The K-sliced kernel (x slice of all rows in shared memory) serves 9 .. 32 rows where it takes the linear and
+// the decode kernels were asked for (the tensor-memory kernel takes the same linears and comes first
+// otherwise): up to eight rows the streaming kernel's batched form is faster (its x fragments from L2 cost
+// less than the K-sliced kernel's accumulation in global memory).
+bool use_rows_kernel(const AilaNf4Linear* l, int64_t ff_pair, int rows) {
+    const int mode = rows_kernel_mode();
     if (mode == 0 || rows < 2 || (mode == 2 && rows <= 8)) return false;
     return nf4::gemv_rows_supported(*l, ff_pair);
 }
@@ -405,45 +427,38 @@ int batched_rows_per_launch(const AilaNf4Linear* l, const AilaNf4Scratch* sc, in
 // bit-identical to the two-phase route and slower at every measured size (each 256-row tile of x pays
 // the dequantisation arithmetic again, and the w tile is produced in step with the tensor core instead
 // of arriving by TMA), so the default is the two-phase route.
-bool use_fused_prefill(const AilaNf4Linear* l, int64_t ff_dim, int seq_len) {
-    static const bool on = [] {
-        const char* e = std::getenv("AILA_NF4_FUSED_PREFILL");
-        return e && e[0] == '1';
-    }();
-    (void)seq_len;
-    if (!on || l->d_cache_bf16) return false;
+bool use_fused_prefill(const AilaNf4Linear* l, int64_t ff_dim) {
+    if (fused_prefill_mode() != 1 || l->d_cache_bf16) return false;
     return nf4::gemm_nf4_fused_supported(*l, ff_dim);
 }
 
 // The tensor-memory kernel serves 9 .. 384 rows in passes of at most 256 rows of equal size
-// (AILA_NF4_MID_ROWS_MIN / _MAX; a maximum below 2 turns it off). Settings that ask for one of the other
-// kernels come first.
+// (AILA_NF4_MID_ROWS_MIN / _MAX; a maximum below 2 turns it off). A setting that asks for one of the other
+// kernels comes first, for the rows that it speaks of: AILA_NF4_DECODE_ROWS_MAX or AILA_NF4_ROWS_KERNEL for
+// small batches, AILA_NF4_FUSED_PREFILL for more rows than those have by default.
 //   From 9 rows on: the four linears of a 2560-wide layer take 54 us against 60 us at 9 rows; at 8 rows the
 //   streaming kernel's batched form is ahead, 52 us against 54 us.
 //   Up to 384 rows: two passes of 150 rows take 137 us for the same linears, dequantise + GEMM about 155 us
 //   for 300 rows; two passes of 256 take 174 us, dequantise + GEMM 165 us for 512.
 int mid_rows_min() {
-    static const int v = [] {
-        const char* e = std::getenv("AILA_NF4_MID_ROWS_MIN");
-        return e && *e ? std::atoi(e) : 9;
-    }();
+    static const int v = env_int("AILA_NF4_MID_ROWS_MIN", 9);
     return v;
 }
 int mid_rows_max() {
-    static const int v = [] {
-        for (const char* name : {"AILA_NF4_DECODE_ROWS_MAX", "AILA_NF4_ROWS_KERNEL", "AILA_NF4_FUSED_PREFILL"}) {
-            const char* o = std::getenv(name);
-            if (o && *o) return 0;
-        }
-        const char* e = std::getenv("AILA_NF4_MID_ROWS_MAX");
-        return e && *e ? std::atoi(e) : 384;
-    }();
+    static const int v = env_int("AILA_NF4_MID_ROWS_MAX", 384);
+    return v;
+}
+
+// Rows up to which a setting asks for the small-batch decode kernels.
+int decode_rows_asked() {
+    static const int v = env_int("AILA_NF4_DECODE_ROWS_MAX", -1) >= 0 || rows_kernel_mode() != 2 ? decode_rows_max() : 0;
     return v;
 }
 
 bool use_mid_rows(const AilaNf4Linear* l, const void* x, int seq_len, int64_t ff_dim) {
     if (seq_len < 2 || seq_len < mid_rows_min() || seq_len > mid_rows_max() || l->d_cache_bf16) return false;
-    if (gemv_kernel_choice() != 0) return false;
+    if (gemv_kernel_choice() != 0 || seq_len <= decode_rows_asked()) return false;
+    if (fused_prefill_mode() >= 0 && seq_len > kDecodeRowsDefault) return false;
     if (reinterpret_cast<uintptr_t>(x) & 15) return false;
     return nf4::gemm_midrows_supported(*l, ff_dim);
 }
@@ -890,7 +905,7 @@ AILA_NF4_API AilaNf4Status aila_nf4_forward(const AilaNf4Linear* l, AilaNf4Scrat
         }
         return AILA_NF4_OK;
     }
-    if (use_fused_prefill(l, 0, seq_len))
+    if (use_fused_prefill(l, 0))
         return nf4::launch_gemm_nf4_fused(*l, x, y, residual, seq_len, 0, sc->sm_count, sc->d_status, s);
     const void* wsrc = l->d_cache_bf16;
     if (!wsrc) {
@@ -947,7 +962,7 @@ AILA_NF4_API AilaNf4Status aila_nf4_forward_gate_up_swiglu(const AilaNf4Linear* 
         }
         return AILA_NF4_OK;
     }
-    if (use_fused_prefill(l, ff_dim, seq_len))
+    if (use_fused_prefill(l, ff_dim))
         return nf4::launch_gemm_nf4_fused(*l, x, out, nullptr, seq_len, ff_dim, sc->sm_count, sc->d_status, s);
     const void* wsrc = l->d_cache_bf16;
     if (!wsrc) {

@@ -45,3 +45,41 @@ def test_launches_overlap_unless_switched_off():
     assert len(names) == 10 and overlapped >= 8, (names, overlapped)   # (all but the first and the dequantisation pass)
     off_names, off = child(OVERLAP, AILA_NF4_PDL="0")
     assert off_names == names and off == 0, (off_names, off)
+
+
+ROUTES = r"""
+import json, re, torch
+from aila_b200 import linear as nf4
+from tests.helpers import captured, make_weight
+lin = nf4.Bnb4BitLinear()
+assert lin.init(make_weight(1, 512, 512), 0), lin.last_error
+sc = nf4.Bnb4BitLinearScratch(0)
+sc.ensure(512, 512, 512, True)
+x, y = (torch.ones(512, 512, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+def route(m):
+    lin.forward(sc, x, y, m)
+    names = [n for n in captured(lambda: lin.forward(sc, x, y, m))[0] if "dequant" not in n]
+    kinds = {re.search("gemv_stream|gemv_rows|gemm_midrows|gemm_bf16_tcgen05_kernelILb[01]", n)[0] for n in names}
+    assert len(kinds) == 1, names
+    return kinds.pop()
+print(json.dumps({m: route(m) for m in (4, 9, 17, 32, 48, 49, 77, 300, 385)}))
+"""
+STREAM, SLICED, MID, GEMM, FUSED = ("gemv_stream", "gemv_rows", "gemm_midrows", "gemm_bf16_tcgen05_kernelILb0",
+                                    "gemm_bf16_tcgen05_kernelILb1")
+
+
+@pytest.mark.parametrize("env,want", [
+    ({}, [STREAM] + [MID] * 7 + [GEMM]),
+    (dict(AILA_NF4_DECODE_ROWS_MAX="17"), [STREAM, SLICED, SLICED, MID, MID, MID, MID, MID, GEMM]),
+    (dict(AILA_NF4_DECODE_ROWS_MAX="48"), [STREAM] + [SLICED] * 4 + [MID] * 3 + [GEMM]),
+    (dict(AILA_NF4_DECODE_ROWS_MAX="0"), [GEMM] + [MID] * 7 + [GEMM]),
+    (dict(AILA_NF4_ROWS_KERNEL="0"), [STREAM] * 5 + [MID] * 3 + [GEMM]),
+    (dict(AILA_NF4_ROWS_KERNEL="1"), [SLICED] * 5 + [MID] * 3 + [GEMM]),
+    (dict(AILA_NF4_ROWS_KERNEL="2"), [STREAM] + [MID] * 7 + [GEMM]),
+    (dict(AILA_NF4_FUSED_PREFILL="0"), [STREAM] + [MID] * 4 + [GEMM] * 4),
+    (dict(AILA_NF4_FUSED_PREFILL="1"), [STREAM] + [MID] * 4 + [FUSED] * 4),
+    (dict(AILA_NF4_MID_ROWS_MIN="49", AILA_NF4_MID_ROWS_MAX="77"), [STREAM] + [SLICED] * 4 + [MID] * 2 + [GEMM] * 2),
+    (dict(AILA_NF4_MID_ROWS_MAX="0"), [STREAM] + [SLICED] * 4 + [GEMM] * 4)],
+    ids=lambda v: "-".join(f"{k[9:]}={n}" for k, n in v.items()) or "default" if isinstance(v, dict) else "")
+def test_settings_choose_the_kernel(env, want):
+    assert list(child(ROUTES, **env).values()) == want
