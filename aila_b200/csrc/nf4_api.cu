@@ -474,14 +474,18 @@ AilaNf4Status run_mid_rows(const AilaNf4Linear* l, AilaNf4Scratch* sc, const voi
         NF4_CUDA(cudaStreamIsCapturing(s, &capture));
         if (capture == cudaStreamCaptureStatusNone && (st = nf4::ensure_mid_partials(sc)) != AILA_NF4_OK) return st;
     }
-    const int passes = (seq_len + nf4::kMidRowsMax - 1) / nf4::kMidRowsMax;
+    // Where the small-batch decode kernels served before (up to 48 rows) the code-book value alone is rounded to
+    // bf16, as they do; above, the weight, as the dequantise + GEMM route does.
+    const bool block_scaled = seq_len <= kDecodeRowsDefault;
+    const int most = block_scaled ? nf4::kMidRowsScaled : nf4::kMidRowsMax;
+    const int passes = (seq_len + most - 1) / most;
     const size_t n_out = (size_t)(ff_dim > 0 ? ff_dim : l->N);
     for (int i = 0, m = 0; i < passes; ++i) {
         const int rows = (seq_len - m + passes - i - 1) / (passes - i);
         st = nf4::launch_gemm_midrows(*l, *sc, static_cast<const char*>(x) + (size_t)m * l->K * 2,
                                       static_cast<char*>(y) + (size_t)m * n_out * 2,
                                       residual ? static_cast<const char*>(residual) + (size_t)m * n_out * 2 : nullptr,
-                                      rows, ff_dim, s);
+                                      rows, ff_dim, block_scaled, s);
         if (st != AILA_NF4_OK) return st;
         m += rows;
     }

@@ -195,11 +195,12 @@ AilaNf4Status launch_gemm_bf16(const void* w_nk, const void* x, void* y, const v
 // nf4_midrows.cu ------------------------------------------------------------------------
 // 2 .. kMidRowsMax rows in one pass over the NF4 units (decoded into tensor memory, no bf16 copy).
 constexpr int kMidRowsMax = 256;
+constexpr int kMidRowsScaled = 32;  // of the block-scaled form: operand bf16(code book), absmax an fp32 factor
 bool gemm_midrows_supported(const AilaNf4Linear& w, int64_t swiglu_ff);
 int gemm_midrows_tiles(const AilaNf4Linear& w, int64_t swiglu_ff);  // counters it needs
 size_t gemm_midrows_partial_bytes(int ctas, int rows);  // of the stream split
 AilaNf4Status ensure_mid_partials(AilaNf4Scratch* sc);
 AilaNf4Status launch_gemm_midrows(const AilaNf4Linear& w, AilaNf4Scratch& sc, const void* x, void* y,
-                                  const void* residual, int rows, int64_t swiglu_ff, cudaStream_t s);
+                                  const void* residual, int rows, int64_t swiglu_ff, bool block_scaled, cudaStream_t s);
 
 }  // namespace nf4

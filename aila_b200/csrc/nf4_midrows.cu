@@ -46,6 +46,7 @@
 
 #include <cstdlib>
 #include <mutex>
+#include <type_traits>
 
 #include "nf4_internal.h"
 #include "nf4_tma.h"
@@ -124,6 +125,20 @@ __device__ __forceinline__ void tmem_st16(uint32_t addr, const uint32_t (&r)[16]
         : "memory");
 }
 
+__device__ __forceinline__ void tmem_ld16(uint32_t addr, float (&v)[16]) {
+    uint32_t r[16];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(addr)
+        : "memory");
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+}
+
 __device__ __forceinline__ void tmem_ld8(uint32_t addr, float (&v)[8]) {
     uint32_t r[8];
     asm volatile(
@@ -171,6 +186,15 @@ __device__ __forceinline__ uint32_t decode2(uint32_t word, uint32_t lut_lane, ui
     return r;
 }
 
+// The same byte as two code-book values rounded to bf16 (block-scaled form).
+template <int I>
+__device__ __forceinline__ uint32_t lookup2(uint32_t word, uint32_t lut_lane) {
+    uint32_t addr, r;
+    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(addr) : "r"(word), "r"(lut_lane), "n"(0x7604 | (I << 4)));
+    asm("ld.shared.u32 %0, [%1];" : "=r"(r) : "r"(addr));
+    return r;
+}
+
 __device__ __forceinline__ uint4 lds_v4(uint32_t a) {
     uint4 v;
     asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
@@ -210,6 +234,9 @@ __device__ __forceinline__ void emit(const MidParams& p, int tile, int quarter, 
     }
 }
 
+// NS = 0: operands bf16(code_book[nibble] * absmax), summed over K in tensor memory. NS = 16 or 32 (the
+// activation rows, rounded up): block-scaled, see the head of the file.
+template <int NS>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_midrows_kernel(const __grid_constant__ CUtensorMap map_x, const MidParams p) {
     extern __shared__ __align__(1024) uint8_t mid_smem[];
@@ -335,7 +362,7 @@ gemm_midrows_kernel(const __grid_constant__ CUtensorMap map_x, const MidParams p
             mbar_init(&done[s], 1);
         }
         for (int b = 0; b < 2; ++b) {
-            mbar_init(&acc_full[b], 1);
+            mbar_init(&acc_full[b], NS > 0 ? kDecodeWarps : 1);
             mbar_init(&acc_empty[b], kDecodeWarps);
         }
         mbar_init(drain, 1);
@@ -350,11 +377,22 @@ gemm_midrows_kernel(const __grid_constant__ CUtensorMap map_x, const MidParams p
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     if (tid < 256) s_nmap[tid] = n_mine;
-    // look-up table: entry e of lane l at e * 256 + l * 8 = {value of e's high nibble, of its low nibble}
-    for (int i = tid; i < 256 * 16; i += kThreads) {  // (whole warps)
-        const int e = i >> 4;
-        const float hi = __shfl_sync(0xffffffffu, q_lane, e >> 4), lo = __shfl_sync(0xffffffffu, q_lane, e & 15);
-        *reinterpret_cast<float4*>(mid_smem + lut_off + (uint32_t)i * 16u) = make_float4(hi, lo, hi, lo);
+    if constexpr (NS > 0) {
+        // look-up table: entry e of lane l at e * 256 + l * 4 = bf16 {value of e's high nibble, of its low nibble}
+        for (int i = tid; i < 256 * 8; i += kThreads) {  // (whole warps)
+            const int e = i >> 3;
+            const float hi = __shfl_sync(0xffffffffu, q_lane, e >> 4), lo = __shfl_sync(0xffffffffu, q_lane, e & 15);
+            const uint32_t w = f32x2_to_bf16x2_bits(hi, lo);
+            *reinterpret_cast<uint4*>(mid_smem + lut_off + (uint32_t)e * 256u + (uint32_t)(i & 7) * 16u) =
+                make_uint4(w, w, w, w);
+        }
+    } else {
+        // look-up table: entry e of lane l at e * 256 + l * 8 = {value of e's high nibble, of its low nibble}
+        for (int i = tid; i < 256 * 16; i += kThreads) {  // (whole warps)
+            const int e = i >> 4;
+            const float hi = __shfl_sync(0xffffffffu, q_lane, e >> 4), lo = __shfl_sync(0xffffffffu, q_lane, e & 15);
+            *reinterpret_cast<float4*>(mid_smem + lut_off + (uint32_t)i * 16u) = make_float4(hi, lo, hi, lo);
+        }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -414,7 +452,7 @@ gemm_midrows_kernel(const __grid_constant__ CUtensorMap map_x, const MidParams p
             for (int left = n; left > 0 && ok; ++seg) {
                 const int b = seg % bufs;
                 const uint32_t d = tmem + (uint32_t)(b * 128);
-                if (seg >= bufs && !wait_spin(&acc_empty[b], ((seg / bufs) - 1) & 1, p.limit, abort_flag)) {
+                if (NS == 0 && seg >= bufs && !wait_spin(&acc_empty[b], ((seg / bufs) - 1) & 1, p.limit, abort_flag)) {
                     give_up(kStatusTimeoutTmem);
                     break;
                 }
@@ -441,10 +479,16 @@ gemm_midrows_kernel(const __grid_constant__ CUtensorMap map_x, const MidParams p
                             if (ok) {
                                 const uint64_t bd = x_desc(base + x_stage(st));
                                 const uint32_t a = tmem + kSlotCol0 + (uint32_t)((set * kGroups + k) * kSlotCols);
+                                if constexpr (NS > 0) {  // a sum of its own for every block
+                                    const uint32_t db = tmem + (uint32_t)((set * kGroups + k) * NS);
 #pragma unroll
-                                for (int j = 0; j < 4; ++j) {
-                                    mma_ts(d, a + 8 * j, bd + 2 * j, p.idesc, acc);
-                                    acc = 1u;
+                                    for (int j = 0; j < 4; ++j) mma_ts(db, a + 8 * j, bd + 2 * j, p.idesc, j > 0);
+                                } else {
+#pragma unroll
+                                    for (int j = 0; j < 4; ++j) {
+                                        mma_ts(d, a + 8 * j, bd + 2 * j, p.idesc, acc);
+                                        acc = 1u;
+                                    }
                                 }
                                 if (p.x_per_item) {
                                     commit(&x_empty[s]);
@@ -462,7 +506,7 @@ gemm_midrows_kernel(const __grid_constant__ CUtensorMap map_x, const MidParams p
                     }
                     commit(&done[set]);
                 }
-                if (ok) commit(&acc_full[b]);
+                if (NS == 0 && ok) commit(&acc_full[b]);
             }
             // no MMA is in flight when tensor and shared memory are given up
             commit(drain);
@@ -470,12 +514,26 @@ gemm_midrows_kernel(const __grid_constant__ CUtensorMap map_x, const MidParams p
         }
         __syncwarp();
     } else if (warp >= kFirstDecodeWarp) {
-        const uint32_t lut_lane = lut + (uint32_t)lane * 8u;
+        const uint32_t lut_lane = lut + (uint32_t)lane * (NS > 0 ? 4u : 8u);
         const uint32_t lane_off = (uint32_t)(quarter * 32) << 16;
         bool ok = true;
         float4 e = e_next;
         int ch = 0;      // chunk
         int c_slot = 0;  // ring slot of the next item
+        // Block-scaled: the lane's row of the CTA's part of the tile, this group's blocks; the absmax of the
+        // blocks whose sums are still to come, of the chunk before (1) and the one before that (2)
+        float acc[NS > 0 ? NS : 1];
+        float am1 = 0.0f, am2 = 0.0f;
+        bool have1 = false, have2 = false;
+        auto add_block = [&](int set, float am) {
+#pragma unroll
+            for (int c0 = 0; c0 < NS; c0 += 16) {
+                float v[16];
+                tmem_ld16(tmem + lane_off + (uint32_t)((set * kGroups + grp) * NS + c0), v);
+#pragma unroll
+                for (int i = 0; i < 16; ++i) acc[c0 + i] = fmaf(am, v[i], acc[c0 + i]);
+            }
+        };
         // the warp's part of one chunk: block kb, or nothing (the chunk is short)
         auto chunk = [&](int kb, bool have) {
             const int set = ch & 1;
@@ -488,6 +546,17 @@ gemm_midrows_kernel(const __grid_constant__ CUtensorMap map_x, const MidParams p
                 }
             }
             ++ch;
+            if constexpr (NS > 0) {
+                if (have2) {  // (its set is this chunk's: both are free again when this warp arrives)
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    add_block(set, am2);
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                }
+                have2 = have1;
+                am2 = am1;
+                have1 = have;
+            }
             if (!have) {
                 if (lane == 0) mbar_arrive(&a_full[set]);
                 return;
@@ -506,28 +575,37 @@ gemm_midrows_kernel(const __grid_constant__ CUtensorMap map_x, const MidParams p
             } else {
                 asm volatile("ld.shared.f32 %0, [%1];" : "=f"(am) : "r"(src + 1024 + 4 * lane));
             }
-            uint64_t am2;
-            asm("mov.b64 %0, {%1, %1};" : "=l"(am2) : "f"(am));
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t dst = tmem + lane_off + kSlotCol0 + (uint32_t)((set * kGroups + grp) * kSlotCols);
             // stored byte 8 t + 2 j + e covers k = 16 j + 4 t + 2 e: operand column 8 j + 2 t + e
             const uint32_t ws[8] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
+            uint64_t am_pair;
+            asm("mov.b64 %0, {%1, %1};" : "=l"(am_pair) : "f"(am));
+            if constexpr (NS > 0) am1 = am;
+            auto pair = [&](auto byte, uint32_t word) {
+                if constexpr (NS > 0) return lookup2<decltype(byte)::value>(word, lut_lane);
+                else return decode2<decltype(byte)::value>(word, lut_lane, am_pair);
+            };
+            using B0 = std::integral_constant<int, 0>;
+            using B1 = std::integral_constant<int, 1>;
+            using B2 = std::integral_constant<int, 2>;
+            using B3 = std::integral_constant<int, 3>;
             uint32_t o[16];
 #pragma unroll
             for (int t = 0; t < 4; ++t) {  // j = 0, 1: the low words of the 8-byte chunks
-                o[2 * t + 0] = decode2<0>(ws[2 * t], lut_lane, am2);
-                o[2 * t + 1] = decode2<1>(ws[2 * t], lut_lane, am2);
-                o[8 + 2 * t + 0] = decode2<2>(ws[2 * t], lut_lane, am2);
-                o[8 + 2 * t + 1] = decode2<3>(ws[2 * t], lut_lane, am2);
+                o[2 * t + 0] = pair(B0{}, ws[2 * t]);
+                o[2 * t + 1] = pair(B1{}, ws[2 * t]);
+                o[8 + 2 * t + 0] = pair(B2{}, ws[2 * t]);
+                o[8 + 2 * t + 1] = pair(B3{}, ws[2 * t]);
             }
             tmem_st16(dst, o);
             uint32_t o2[16];
 #pragma unroll
             for (int t = 0; t < 4; ++t) {  // j = 2, 3: the high words
-                o2[2 * t + 0] = decode2<0>(ws[2 * t + 1], lut_lane, am2);
-                o2[2 * t + 1] = decode2<1>(ws[2 * t + 1], lut_lane, am2);
-                o2[8 + 2 * t + 0] = decode2<2>(ws[2 * t + 1], lut_lane, am2);
-                o2[8 + 2 * t + 1] = decode2<3>(ws[2 * t + 1], lut_lane, am2);
+                o2[2 * t + 0] = pair(B0{}, ws[2 * t + 1]);
+                o2[2 * t + 1] = pair(B1{}, ws[2 * t + 1]);
+                o2[8 + 2 * t + 0] = pair(B2{}, ws[2 * t + 1]);
+                o2[8 + 2 * t + 1] = pair(B3{}, ws[2 * t + 1]);
             }
             tmem_st16(dst + 16, o2);
             fetch();  // (every lane has used the slot's words: tcgen05.st is warp-wide)
@@ -548,11 +626,44 @@ gemm_midrows_kernel(const __grid_constant__ CUtensorMap map_x, const MidParams p
             const int le = min(n, ls + KB - kb0);  // this CTA's part of the tile: local items [ls, le)
             e = e_next;
             if (le < n) e_next = row_scale(tile + 1);
+            if constexpr (NS > 0) {
+#pragma unroll
+                for (int i = 0; i < NS; ++i) acc[i] = 0.0f;
+            }
             for (int j = grp; j < (le - ls + kGroups - 1) / kGroups * kGroups && ok; j += kGroups) chunk(kb0 + j, j < le - ls);
             if (!ok) break;
+            if constexpr (NS > 0) {
+                // ---- the last blocks' sums; the group's row to tensor memory, where the groups meet ----
+#pragma unroll
+                for (int back = 2; back > 0; --back) {
+                    if ((back == 2 ? have2 : have1) && ok) {
+                        const int c0 = ch - back;
+                        ok = wait_spin(&done[c0 & 1], (c0 >> 1) & 1, p.limit, abort_flag);
+                        ok = __all_sync(0xffffffffu, ok);
+                        if (ok) {
+                            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                            add_block(c0 & 1, back == 2 ? am2 : am1);
+                        }
+                    }
+                }
+                have1 = have2 = false;
+                if (ok) {
+#pragma unroll
+                    for (int c0 = 0; c0 < NS; c0 += 16) {
+                        uint32_t r[16];
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) r[i] = __float_as_uint(acc[c0 + i]);
+                        tmem_st16(tmem + lane_off + (uint32_t)(grp * NS + c0), r);
+                    }
+                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&acc_full[0]);
+                }
+            }
             // ---- drain the accumulator ----
-            const int b = seg % bufs;
-            ok = wait_spin(&acc_full[b], (seg / bufs) & 1, p.limit, abort_flag);
+            const int b = NS > 0 ? 0 : seg % bufs;
+            if (ok) ok = wait_spin(&acc_full[b], (NS > 0 ? seg : seg / bufs) & 1, p.limit, abort_flag);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) {
                 if (lane == 0) give_up(kStatusTimeoutTmem);
@@ -565,12 +676,24 @@ gemm_midrows_kernel(const __grid_constant__ CUtensorMap map_x, const MidParams p
                 waited = true;
             }
             const uint32_t dcol = tmem + lane_off + (uint32_t)(b * 128);
+            auto sums8 = [&](int ch8, float (&v)[8]) {  // eight columns of the lane's row
+                tmem_ld8(dcol + (uint32_t)(ch8 * 8), v);
+                if constexpr (NS > 0) {
+#pragma unroll
+                    for (int g = 1; g < kGroups; ++g) {
+                        float w[8];
+                        tmem_ld8(dcol + (uint32_t)(g * NS + ch8 * 8), w);
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) v[i] += w[i];
+                    }
+                }
+            };
             const bool whole = kb0 == 0 && le - ls == KB;
             const size_t part = (size_t)kTileM * p.NB;
             if (p.split <= 1 && whole) {
                 for (int ch = grp; ch < chunks; ch += kGroups) {
                     float v[8];
-                    tmem_ld8(dcol + (uint32_t)(ch * 8), v);
+                    sums8(ch, v);
                     emit(p, tile, quarter, lane, ch * 8, v);
                     __syncwarp();  // (lanes past the output left early; the next load is warp-wide)
                 }
@@ -581,7 +704,7 @@ gemm_midrows_kernel(const __grid_constant__ CUtensorMap map_x, const MidParams p
                                         : reinterpret_cast<float4*>(p.partials + ((size_t)c * 2 + (kb0 == 0 ? 1 : 0)) * part);
                 for (int ch = grp; ch < chunks; ch += kGroups) {
                     float v[8];
-                    tmem_ld8(dcol + (uint32_t)(ch * 8), v);
+                    sums8(ch, v);
                     float4* at = o + (size_t)ch * 2 * kTileM + row;
                     at[0] = make_float4(v[0], v[1], v[2], v[3]);
                     at[kTileM] = make_float4(v[4], v[5], v[6], v[7]);
@@ -589,7 +712,7 @@ gemm_midrows_kernel(const __grid_constant__ CUtensorMap map_x, const MidParams p
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
-            if (lane == 0) mbar_arrive(&acc_empty[b]);
+            if (NS == 0 && lane == 0) mbar_arrive(&acc_empty[b]);
             if (p.split == 0 && !whole) {
                 const int t0 = tile * KB, t1 = t0 + KB - 1;  // first and last item of the tile
                 const int big = r * (q + 1);
@@ -685,6 +808,8 @@ gemm_midrows_kernel(const __grid_constant__ CUtensorMap map_x, const MidParams p
     }
 }
 
+using MidKernel = void (*)(const CUtensorMap, const MidParams);
+
 // What the launches on one device need to know, found out once.
 struct MidDevice {
     cudaError_t err = cudaSuccess;
@@ -696,7 +821,9 @@ const MidDevice& mid_device(int dev) {
     static std::once_flag once[64];
     MidDevice& d = devs[dev];
     std::call_once(once[dev], [&] {
-        d.err = cudaFuncSetAttribute(gemm_midrows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+        for (MidKernel k : {gemm_midrows_kernel<0>, gemm_midrows_kernel<16>, gemm_midrows_kernel<32>})
+            if (d.err == cudaSuccess)
+                d.err = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
         for (int s = 1; s <= 8 && d.err == cudaSuccess; ++s) {
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3((unsigned)(s * 148));
@@ -708,7 +835,7 @@ const MidDevice& mid_device(int dev) {
             attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
             cfg.attrs = attr;
             cfg.numAttrs = 1;
-            d.err = cudaOccupancyMaxActiveClusters(&d.clusters[s], gemm_midrows_kernel, &cfg);
+            d.err = cudaOccupancyMaxActiveClusters(&d.clusters[s], gemm_midrows_kernel<0>, &cfg);
         }
     });
     return d;
@@ -757,7 +884,9 @@ size_t gemm_midrows_partial_bytes(int ctas, int rows) {
 
 // x is 16-byte aligned; rows <= kMidRowsMax; counters hold a zero per tile.
 AilaNf4Status launch_gemm_midrows(const AilaNf4Linear& w, AilaNf4Scratch& sc, const void* x, void* y,
-                                  const void* residual, int rows, int64_t swiglu_ff, cudaStream_t s) {
+                                  const void* residual, int rows, int64_t swiglu_ff, bool block_scaled, cudaStream_t s) {
+    if (rows < 1 || rows > (block_scaled ? kMidRowsScaled : kMidRowsMax))
+        return fail(AILA_NF4_ERR_INVALID_ARGUMENT, "gemm_midrows: row count");
     MidParams p = {};
     const ScaleParams sp = w.scale_params();
     p.units = w.d_units;
@@ -817,7 +946,10 @@ AilaNf4Status launch_gemm_midrows(const AilaNf4Linear& w, AilaNf4Scratch& sc, co
         attr[cfg.numAttrs].val.clusterDim.y = attr[cfg.numAttrs].val.clusterDim.z = 1;
         ++cfg.numAttrs;
     }
-    const cudaError_t le = cudaLaunchKernelEx(&cfg, gemm_midrows_kernel, map_x, p);
+    const MidKernel kernel = !block_scaled ? gemm_midrows_kernel<0>
+                             : rows <= 16  ? gemm_midrows_kernel<16>
+                                           : gemm_midrows_kernel<32>;
+    const cudaError_t le = cudaLaunchKernelEx(&cfg, kernel, map_x, p);
     if (le != cudaSuccess) return cuda_fail(le, "gemm_midrows_kernel launch");
     return AILA_NF4_OK;
 }

@@ -1,7 +1,10 @@
 """The tensor-memory kernel behind aila_nf4_forward / aila_nf4_forward_gate_up_swiglu for a few to a few
-hundred rows, against the bit-exact dequantised weight in float64. With the weights equal, what is left is
-the order of an fp32 sum and the rounding of the result to bf16 (8 significant bits: at most 2^-8 of the
-value; twice more where gate and up pass through bf16)."""
+hundred rows, against its weights in float64: above 48 rows the bit-exact dequantised weight, up to 48 rows
+the code-book value rounded to bf16 times the fp32 absmax, which is what the small-batch decode kernels
+multiply by and closer to the unrounded weight. With the weights equal, what is left is the order of an fp32
+sum and the rounding of the result to bf16 (8 significant bits: at most 2^-8 of the value; twice more where
+gate and up pass through bf16)."""
+import numpy as np
 import pytest
 import torch
 
@@ -27,6 +30,17 @@ def _linear(nf4, *args):
     return l
 
 
+def _weight(lin, tensors, m):
+    """[in_features, out_features] in float64: what a call of m rows multiplies by."""
+    if m > 48:
+        return lin.dequantize_weight().double()
+    code = torch.from_numpy(np.asarray(tensors[0].quant_map, np.float32)).cuda().to(torch.bfloat16).double()
+    packed = torch.from_numpy(np.concatenate([t.packed for t in tensors])).cuda()
+    nibbles = torch.stack((packed >> 4, packed & 15), dim=1).view(lin.out_features(), -1, tensors[0].blocksize)
+    absmax = lin.expand_absmax(tensors[0].blocksize).double()
+    return (code[nibbles.int()] * absmax.unsqueeze(2)).view(lin.out_features(), -1).T
+
+
 def _x(seed, m, k):
     return torch.randn(m, k, generator=torch.Generator().manual_seed(seed)).to(torch.bfloat16).cuda()
 
@@ -41,7 +55,7 @@ def _x(seed, m, k):
 @pytest.mark.parametrize("m", [9, 16, 17, 77, 96, 97, 128, 129, 256, 257, 384])
 def test_linear(nf4, scratch, n, k, blocksize, nested, m):
     lin = _linear(nf4, 31 + n, n, k, blocksize, nested)
-    w = lin.dequantize_weight().double()
+    w = _weight(lin, [make_weight(31 + n, n, k, blocksize, nested)], m)
     x, res = _x(m, m, k), _x(m + 1, m, n)
     y = torch.full((m + 1, n), 7.0, dtype=torch.bfloat16, device="cuda")
     first = None
@@ -57,13 +71,45 @@ def test_linear(nf4, scratch, n, k, blocksize, nested, m):
     scratch.check()
 
 
+@pytest.mark.parametrize("n,k,blocksize,nested", [
+    (16, 64, 64, True), (100, 448, 64, False), (129, 1024, 256, True), (1000, 9728, 64, True),
+    (6144, 2560, 64, True), (40000, 128, 128, False)])
+@pytest.mark.parametrize("m", [31, 32, 33, 47, 48, 49])
+def test_linear_at_the_edges_of_the_block_scaled_form(nf4, scratch, n, k, blocksize, nested, m):
+    """Its one pass of 32 rows, two passes, and the first row count of the other form."""
+    test_linear(nf4, scratch, n, k, blocksize, nested, m)
+
+
+def test_absmax_is_not_rounded_up_to_48_rows(nf4, scratch):
+    """A code of +-1 is the block's absmax itself: with only such codes and one block per row the result is
+    absmax times a sum of x that fp32 holds exactly, rounded once."""
+    from aila_b200 import synth
+    n, k = 512, 64
+    gen = torch.Generator().manual_seed(3)
+    absmax = torch.rand(n, generator=gen) + 0.5
+    signs = torch.randint(2, (n, k), generator=gen)
+    quant_map = synth.nf4_codebook()
+    assert quant_map[0] == -1 and quant_map[15] == 1
+    codes = (signs * 15).to(torch.uint8)
+    packed = ((codes[:, 0::2] << 4) | codes[:, 1::2]).reshape(-1).numpy()
+    lin = nf4.Bnb4BitLinear()
+    assert lin.init(synth.Nf4Tensors(n, k, 64, packed, None, absmax.numpy(), quant_map, None, None), 0), lin.last_error
+    for m in (9, 32, 40):
+        x = torch.randint(-128, 128, (m, k), generator=gen).to(torch.bfloat16)   # |sums| <= 2^13: exact
+        y = torch.empty(m, n, dtype=torch.bfloat16, device="cuda")
+        lin.forward(scratch, x.cuda(), y, m)
+        sums = x.double() @ (2 * signs - 1).double().T
+        want = (absmax * sums.float()).to(torch.bfloat16)
+        assert torch.equal(y.cpu(), want)
+
+
 @pytest.mark.parametrize("ff,k", [(16, 64), (80, 448), (1040, 512), (9728, 2560)])
 @pytest.mark.parametrize("m", [9, 31, 77, 200, 300])
 def test_gate_up(nf4, scratch, ff, k, m):
     g, u = _linear(nf4, 5, ff, k), _linear(nf4, 6, ff, k)
     f = nf4.Bnb4BitLinear()
     assert f.init_fused_rows(g, u), f.last_error
-    w = f.dequantize_weight().double()
+    w = _weight(f, [make_weight(5, ff, k), make_weight(6, ff, k)], m)
     x = _x(m, m, k)
     out = torch.full((m + 1, ff), 7.0, dtype=torch.bfloat16, device="cuda")
     assert nf4.Bnb4BitLinear.try_forward_decode_gate_up_swiglu(f, scratch, x, out[:m], ff, m)
