@@ -440,6 +440,11 @@ bool use_fused_prefill(const AilaNf4Linear* l, int64_t ff_dim) {
 //   streaming kernel's batched form is ahead, 52 us against 54 us.
 //   Up to 384 rows: two passes of 150 rows take 137 us for the same linears, dequantise + GEMM about 155 us
 //   for 300 rows; two passes of 256 take 174 us, dequantise + GEMM 165 us for 512.
+// Within these rows it does not take (mid_rows_pay; us on this kernel and on the route that serves instead)
+//   more row tiles than SMs with a short K, where setting up and finishing a tile outweighs its blocks:
+//   60000x256 at 128 rows 24.1 / 18.0; up to 16 rows 30000x512 11.0 / 9.4, but 30000x1024 14.6 / 15.8;
+//   two passes with a short K (8192x1024 at 320 rows 16.6 / 15.3, 30000x512 31.9 / 23.4, but 16384x1536
+//   25.9 / 34.4), unless the bf16 copy that the GEMM would read is larger than L2 (151936x1024 164 / 191).
 int mid_rows_min() {
     static const int v = env_int("AILA_NF4_MID_ROWS_MIN", 9);
     return v;
@@ -455,12 +460,18 @@ int decode_rows_asked() {
     return v;
 }
 
-bool use_mid_rows(const AilaNf4Linear* l, const void* x, int seq_len, int64_t ff_dim) {
+bool mid_rows_pay(const AilaNf4Linear* l, int seq_len, int64_t ff_dim, int sm_count) {
+    if (nf4::gemm_midrows_tiles(*l, ff_dim) > sm_count && l->K < (seq_len <= 16 ? 1024 : 512)) return false;
+    const bool copy_beyond_l2 = l->N * l->K * 2 > (int64_t)126 << 20;
+    return seq_len <= nf4::kMidRowsMax || l->K >= 1536 || (l->K >= 1024 && copy_beyond_l2);
+}
+
+bool use_mid_rows(const AilaNf4Linear* l, const AilaNf4Scratch* sc, const void* x, int seq_len, int64_t ff_dim) {
     if (seq_len < 2 || seq_len < mid_rows_min() || seq_len > mid_rows_max() || l->d_cache_bf16) return false;
     if (gemv_kernel_choice() != 0 || seq_len <= decode_rows_asked()) return false;
     if (fused_prefill_mode() >= 0 && seq_len > kDecodeRowsDefault) return false;
     if (reinterpret_cast<uintptr_t>(x) & 15) return false;
-    return nf4::gemm_midrows_supported(*l, ff_dim);
+    return nf4::gemm_midrows_supported(*l, ff_dim) && mid_rows_pay(l, seq_len, ff_dim, sc->sm_count);
 }
 
 AilaNf4Status run_mid_rows(const AilaNf4Linear* l, AilaNf4Scratch* sc, const void* x, void* y, const void* residual,
@@ -891,7 +902,7 @@ AILA_NF4_API AilaNf4Status aila_nf4_forward(const AilaNf4Linear* l, AilaNf4Scrat
     if (guard.err != cudaSuccess) return nf4::cuda_fail(guard.err, "cudaSetDevice");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (seq_len == 1) return run_decode(l, sc, x, y, residual, 0, s);
-    if (use_mid_rows(l, x, seq_len, 0)) return run_mid_rows(l, sc, x, y, residual, seq_len, 0, s);
+    if (use_mid_rows(l, sc, x, seq_len, 0)) return run_mid_rows(l, sc, x, y, residual, seq_len, 0, s);
     if (use_batched_decode(l, sc, x, seq_len, 0)) {
         // a few rows: the batched decode kernel carries up to 32 rows through the tensor-core
         // tile's batch columns (every decoded weight fragment feeds one operation per block of
@@ -936,7 +947,7 @@ AILA_NF4_API AilaNf4Status aila_nf4_forward_gate_up_swiglu(const AilaNf4Linear* 
     if (guard.err != cudaSuccess) return nf4::cuda_fail(guard.err, "cudaSetDevice");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (seq_len == 1) return run_decode(l, sc, x, out, nullptr, ff_dim, s);
-    if (use_mid_rows(l, x, seq_len, ff_dim)) return run_mid_rows(l, sc, x, out, nullptr, seq_len, ff_dim, s);
+    if (use_mid_rows(l, sc, x, seq_len, ff_dim)) return run_mid_rows(l, sc, x, out, nullptr, seq_len, ff_dim, s);
     if (seq_len > 8 && !use_rows_kernel(l, ff_dim, seq_len) && use_batched_decode(l, sc, x, seq_len, 0) &&
         batched_rows_per_launch(l, sc, 0, seq_len) > 8) {
         // more than eight rows: the unpaired batched kernel over the fused rows (one pass over the

@@ -841,23 +841,48 @@ const MidDevice& mid_device(int dev) {
     return d;
 }
 
-// Time model in items of one (row tile, 64-block): waves x (items of a CTA + what finishing a tile
-// costs). 0: the stream split.
-int choose_split(const MidDevice& d, int n_tiles, int KB, int NB, int sm_count) {
+// Time of a launch among others in us, by split: constants of a straight-line fit to 31 shapes (256x512 to
+// 151936x1024, 5120x8192, gate|up up to 51200x5120) times 13 row counts, every split forced, on 148 SMs.
+// `col` constants are per 100 activation rows (rounded up to 16); a chunk is up to four 64-blocks.
+struct SplitCost {
+    // clusters: per chunk of a CTA, per wave of tiles (whole tiles; shared by a cluster), launches that
+    // cannot share the chip with the next one, waves behind the first
+    double chunk, chunk_col, one, one_col, many, many_col, alone, wave;
+    // stream: per chunk, per tile of a CTA, per CTA of a tile behind the second, launch, not shared
+    double s_chunk, s_chunk_col, tile, tile_col, join, join_col, launch, launch_col, s_alone;
+};
+constexpr SplitCost kCostScaled = {0.66, 0.68, 2.08, 1.40, 2.97, 2.77, 1.63, 1.77,
+                                   0.97, 1.69, 0.74, 0.23, 0.15, 0.07, 2.05, 2.26, 3.92};
+constexpr SplitCost kCostPlain = {0.78, 0.21, 1.29, 1.66, 2.51, 1.84, 1.83, 2.17,
+                                  1.00, 0.57, 0.68, 0.53, 0.00, 0.57, 0.52, 2.50, 5.48};
+
+// 0: the stream split; else CTAs per tile. On the measured shapes the choice is 0.4 % behind the best split on
+// average and 10 % at worst (10 % on average and 57 % at worst by the model of one layer's width before it:
+// 6144x2560 at 32 rows 14.9 -> 9.5 us, 30000x512 at 256 rows 30.2 -> 20.4 us).
+int choose_split(const MidDevice& d, int n_tiles, int KB, int NB, bool block_scaled, int sm_count) {
     static const int forced = [] {  // for measurements: AILA_NF4_MID_SPLIT=0..8
         const char* e = std::getenv("AILA_NF4_MID_SPLIT");
         return e && *e ? std::atoi(e) : -1;
     }();
     if (forced >= 0 && forced <= 8 && forced <= KB) return forced;
-    const double wide = NB / 80.0;
+    const SplitCost& c = block_scaled ? kCostScaled : kCostPlain;
+    const double cols = NB / 100.0;
     const int64_t total = (int64_t)n_tiles * KB;
-    const double ctas = (double)(total / 8 < sm_count ? (total / 8 > 0 ? total / 8 : 1) : sm_count);
-    double best = total / ctas + 10.0 + (4.0 + 2.0 * KB * ctas / total) * wide;
+    const int64_t ctas = (total + 7) / 8 < sm_count ? (total + 7) / 8 : sm_count;
+    const double items = (double)total / ctas, tiles = items / KB;
+    double best = 1e30;
     int split = 0;
+    if (ctas <= 8 * (int64_t)n_tiles)  // (a tile's last CTA adds all parts: not more than a cluster has)
+        best = items / 4 * (c.s_chunk + c.s_chunk_col * cols) + tiles * (c.tile + c.tile_col * cols) +
+               (1 / tiles > 2 ? (1 / tiles - 2) * (c.join + c.join_col * cols) : 0) + c.launch + c.launch_col * cols +
+               (2 * ctas > sm_count ? c.s_alone : 0);
     for (int s = 1; s <= 8 && s <= KB; ++s) {
         if (d.clusters[s] <= 0) continue;
         const int waves = (n_tiles + d.clusters[s] - 1) / d.clusters[s];
-        const double cost = waves * ((KB + s - 1) / s + 6.0 + (s > 1 ? 3.0 + 4.0 * wide : 2.0 * wide));
+        const int chunks = ((KB + s - 1) / s + kGroups - 1) / kGroups;
+        const double cost = waves * (chunks * (c.chunk + c.chunk_col * cols) +
+                                     (s == 1 ? c.one + c.one_col * cols : c.many + c.many_col * cols)) +
+                            (2 * n_tiles > d.clusters[s] ? c.alone : 0) + (waves - 1) * c.wave;
         if (cost < best) {
             best = cost;
             split = s;
@@ -920,7 +945,7 @@ AilaNf4Status launch_gemm_midrows(const AilaNf4Linear& w, AilaNf4Scratch& sc, co
     cudaGetDevice(&dev);
     const MidDevice& md = mid_device(dev & 63);
     if (md.err != cudaSuccess) return cuda_fail(md.err, "cudaFuncSetAttribute(gemm_midrows)");
-    p.split = choose_split(md, p.n_tiles, p.KU, p.NB, sc.sm_count);
+    p.split = choose_split(md, p.n_tiles, p.KU, p.NB, block_scaled, sc.sm_count);
     const int64_t total = (int64_t)p.n_tiles * p.KU;
     const int64_t want = p.split > 0 ? (int64_t)p.n_tiles * p.split : (total + 7) / 8;  // stream: eight items per CTA at least
     const int grid = (int)(p.split > 0 || want < sc.sm_count ? want : sc.sm_count);

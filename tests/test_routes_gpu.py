@@ -52,10 +52,10 @@ import json, re, torch
 from aila_b200 import linear as nf4
 from tests.helpers import captured, make_weight
 lin = nf4.Bnb4BitLinear()
-assert lin.init(make_weight(1, 512, 512), 0), lin.last_error
+assert lin.init(make_weight(1, 512, 2048), 0), lin.last_error
 sc = nf4.Bnb4BitLinearScratch(0)
-sc.ensure(512, 512, 512, True)
-x, y = (torch.ones(512, 512, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+sc.ensure(512, 2048, 512, True)
+x, y = (torch.ones(512, k, dtype=torch.bfloat16, device="cuda") for k in (2048, 512))
 def route(m):
     lin.forward(sc, x, y, m)
     names = [n for n in captured(lambda: lin.forward(sc, x, y, m))[0] if "dequant" not in n]
@@ -83,3 +83,34 @@ STREAM, SLICED, MID, GEMM, FUSED = ("gemv_stream", "gemv_rows", "gemm_midrows", 
     ids=lambda v: "-".join(f"{k[9:]}={n}" for k, n in v.items()) or "default" if isinstance(v, dict) else "")
 def test_settings_choose_the_kernel(env, want):
     assert list(child(ROUTES, **env).values()) == want
+
+
+@pytest.mark.parametrize("n,k,rows,want", [
+    (18944, 256, (9, 49, 256), [MID] * 3), (18945, 256, (9, 49, 256), [SLICED, GEMM, GEMM]),
+    (18945, 448, (48,), [SLICED]), (18945, 512, (16, 17, 256, 257), [SLICED, MID, MID, GEMM]),
+    (18945, 960, (16, 384), [SLICED, GEMM]), (18945, 1024, (9, 384), [MID, GEMM]),
+    (512, 1472, (256, 257), [MID, GEMM]), (512, 1536, (256, 257), [MID, MID]), (65536, 1024, (384,), [MID])])
+def test_shapes_choose_the_kernel(n, k, rows, want):
+    """Both sides of every line of the rule, 148 tiles of 128 rows and one more among them."""
+    import re
+
+    import torch
+
+    from aila_b200 import linear as nf4, synth
+    from tests.helpers import captured
+    packed = torch.randint(256, (n * k // 2,), dtype=torch.uint8).numpy()
+    w = synth.Nf4Tensors(n, k, 64, packed, None, torch.ones(n * k // 64).numpy(), synth.nf4_codebook(), None, None)
+    lin = nf4.Bnb4BitLinear()
+    assert lin.init(w, 0), lin.last_error
+    sc = nf4.Bnb4BitLinearScratch(0)
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("sizes for 148 SMs")
+    got = []
+    for m in rows:
+        x, y = (torch.zeros(m, c, dtype=torch.bfloat16, device="cuda") for c in (k, n))
+        lin.forward(sc, x, y, m)
+        names = captured(lambda: lin.forward(sc, x, y, m))[0]
+        got.append(re.search("gemv_stream|gemv_rows|gemm_midrows|gemm_bf16_tcgen05_kernelILb[01]", names[-1])[0])
+    assert got == want
+    lin.close()
+    sc.close()
