@@ -442,7 +442,8 @@ bool use_fused_prefill(const AilaNf4Linear* l, int64_t ff_dim) {
 //   for 300 rows; two passes of 256 take 174 us, dequantise + GEMM 165 us for 512.
 // Within these rows it does not take (mid_rows_pay; us on this kernel and on the route that serves instead)
 //   more row tiles than SMs with a short K, where setting up and finishing a tile outweighs its blocks:
-//   60000x256 at 128 rows 24.1 / 18.0; up to 16 rows 30000x512 11.0 / 9.4, but 30000x1024 14.6 / 15.8;
+//   60000x256 at 128 rows 24.1 / 18.0, but 15.0 / 18.2 at 24; up to 16 rows 30000x512 11.0 / 9.4, but 30000x1024
+//   14.6 / 15.8;
 //   two passes with a short K (8192x1024 at 320 rows 16.6 / 15.3, 30000x512 31.9 / 23.4, but 16384x1536
 //   25.9 / 34.4), unless the bf16 copy that the GEMM would read is larger than L2 (151936x1024 164 / 191).
 int mid_rows_min() {
@@ -461,7 +462,8 @@ int decode_rows_asked() {
 }
 
 bool mid_rows_pay(const AilaNf4Linear* l, int seq_len, int64_t ff_dim, int sm_count) {
-    if (nf4::gemm_midrows_tiles(*l, ff_dim) > sm_count && l->K < (seq_len <= 16 ? 1024 : 512)) return false;
+    if (nf4::gemm_midrows_tiles(*l, ff_dim) > sm_count && l->K < (seq_len <= 16 ? 1024 : seq_len <= kDecodeRowsDefault ? 256 : 512))
+        return false;
     const bool copy_beyond_l2 = l->N * l->K * 2 > (int64_t)126 << 20;
     return seq_len <= nf4::kMidRowsMax || l->K >= 1536 || (l->K >= 1024 && copy_beyond_l2);
 }
@@ -485,8 +487,8 @@ AilaNf4Status run_mid_rows(const AilaNf4Linear* l, AilaNf4Scratch* sc, const voi
         NF4_CUDA(cudaStreamIsCapturing(s, &capture));
         if (capture == cudaStreamCaptureStatusNone && (st = nf4::ensure_mid_partials(sc)) != AILA_NF4_OK) return st;
     }
-    // Where the small-batch decode kernels served before (up to 48 rows) the code-book value alone is rounded to
-    // bf16, as they do; above, the weight, as the dequantise + GEMM route does.
+    // Up to 48 rows, where the small-batch decode kernels serve otherwise, the code-book value alone is rounded to
+    // bf16, as there; above, the weight, as on the dequantise + GEMM route.
     const bool block_scaled = seq_len <= kDecodeRowsDefault;
     const int most = block_scaled ? nf4::kMidRowsScaled : nf4::kMidRowsMax;
     const int passes = (seq_len + most - 1) / most;

@@ -195,7 +195,7 @@ AilaNf4Status launch_gemm_bf16(const void* w_nk, const void* x, void* y, const v
 // nf4_midrows.cu ------------------------------------------------------------------------
 // 2 .. kMidRowsMax rows in one pass over the NF4 units (decoded into tensor memory, no bf16 copy).
 constexpr int kMidRowsMax = 256;
-constexpr int kMidRowsScaled = 32;  // of the block-scaled form: operand bf16(code book), absmax an fp32 factor
+constexpr int kMidRowsScaled = 48;  // of the block-scaled form: operand bf16(code book), absmax an fp32 factor
 bool gemm_midrows_supported(const AilaNf4Linear& w, int64_t swiglu_ff);
 int gemm_midrows_tiles(const AilaNf4Linear& w, int64_t swiglu_ff);  // counters it needs
 size_t gemm_midrows_partial_bytes(int ctas, int rows);  // of the stream split

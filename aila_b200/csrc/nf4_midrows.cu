@@ -1,5 +1,14 @@
 // A few to a few hundred activation rows: y[M][N] = x[M][K] * W[N][K]^T straight from the NF4 units,
-// one pass over the weights, no bf16 copy of W in memory.
+// one pass over the weights, no bf16 copy of W in memory. Two forms of one kernel:
+//   NS = 0   (49 rows and more) operand bf16(code_book[nibble] * absmax), sums over K in tensor memory: the
+//            weights of the dequantise + GEMM route
+//   NS > 0   (up to 16, 32 or 48 rows) block-scaled: operand bf16(code_book[nibble]), every 64-block's sum by
+//            itself in tensor memory, times the fp32 absmax added up in registers: the arithmetic of the
+//            small-batch decode kernels. A decode thread adds up a quarter of its row's columns (the group's),
+//            so it needs the absmax of all four blocks of a chunk: through the unused half of the table's
+//            lines. Block sums have two sets of tensor-memory columns up to 32 rows, one at 48. (With all
+//            columns of the group's own block per thread the loop spilled, and 33..48 rows took two passes:
+//            twelve layers at 32 rows 643 us against 584, down at 40 rows 24.5 against 13.4.)
 //
 // The weight is the A operand of tcgen05.mma and lives in TENSOR MEMORY: a decode thread owns one
 // output row of a 128-row tile, reads the row's 32 nibble bytes of a 64-wide block (coalesced: a
@@ -67,6 +76,7 @@ constexpr int kMaxX = kSets * kGroups;   // blocks of x in the ring at most
 constexpr uint32_t kLutBytes = 65536u;   // look-up table, at the first shared address that is a multiple of 64 KB
 constexpr uint32_t kXRing = 131072u;     // the x ring behind it starts here at the latest, counted from the CTA's first byte
 constexpr uint32_t kPart = 65536u;       // a cluster's partial tiles, at the same place in every CTA
+constexpr uint32_t kPartScaled = 131072u;  // the same in the block-scaled form (the table's lines hold absmax values)
 constexpr int kSmem = 227 * 1024;
 constexpr int kHeadBytes = 2048;         // barriers, code books
 constexpr int kDepth = 3;                // items a decode warp has in flight
@@ -125,18 +135,25 @@ __device__ __forceinline__ void tmem_st16(uint32_t addr, const uint32_t (&r)[16]
         : "memory");
 }
 
-__device__ __forceinline__ void tmem_ld16(uint32_t addr, float (&v)[16]) {
-    uint32_t r[16];
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n\t"
-        "tcgen05.wait::ld.sync.aligned;"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(addr)
-        : "memory");
+// Four or eight columns without a wait: the values are there after tmem_landed() on them.
+__device__ __forceinline__ void tmem_ld_start(uint32_t addr, uint32_t* r, std::integral_constant<int, 4>) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void tmem_ld_start(uint32_t addr, uint32_t* r, std::integral_constant<int, 8>) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void tmem_ld_start(uint32_t addr, uint32_t* r, std::integral_constant<int, 12>) {
+    tmem_ld_start(addr, r, std::integral_constant<int, 8>{});
+    tmem_ld_start(addr + 8, r + 8, std::integral_constant<int, 4>{});
+}
+template <int N>
+__device__ __forceinline__ void tmem_landed(uint32_t (&r)[N]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+    for (int i = 0; i < N; ++i) asm volatile("" : "+r"(r[i]));  // (no use before the wait)
 }
 
 __device__ __forceinline__ void tmem_ld8(uint32_t addr, float (&v)[8]) {
@@ -234,12 +251,14 @@ __device__ __forceinline__ void emit(const MidParams& p, int tile, int quarter, 
     }
 }
 
-// NS = 0: operands bf16(code_book[nibble] * absmax), summed over K in tensor memory. NS = 16 or 32 (the
+// NS = 0: operands bf16(code_book[nibble] * absmax), summed over K in tensor memory. NS = 16, 32 or 48 (the
 // activation rows, rounded up): block-scaled, see the head of the file.
 template <int NS>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_midrows_kernel(const __grid_constant__ CUtensorMap map_x, const MidParams p) {
     extern __shared__ __align__(1024) uint8_t mid_smem[];
+    constexpr int kSumSets = NS <= 32 ? 2 : 1;  // sets of block sums in tensor memory (256 columns)
+    constexpr int C = NS > 0 ? NS / kGroups : 8;  // block-scaled: columns of a row that a decode thread adds up
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const uint32_t base = smem_u32(mid_smem);
     // The table's lines are found by inserting a byte into an address, so it starts at a multiple of 64 KB of
@@ -362,7 +381,7 @@ gemm_midrows_kernel(const __grid_constant__ CUtensorMap map_x, const MidParams p
             mbar_init(&done[s], 1);
         }
         for (int b = 0; b < 2; ++b) {
-            mbar_init(&acc_full[b], NS > 0 ? kDecodeWarps : 1);
+            mbar_init(&acc_full[b], 1);
             mbar_init(&acc_empty[b], kDecodeWarps);
         }
         mbar_init(drain, 1);
@@ -480,7 +499,7 @@ gemm_midrows_kernel(const __grid_constant__ CUtensorMap map_x, const MidParams p
                                 const uint64_t bd = x_desc(base + x_stage(st));
                                 const uint32_t a = tmem + kSlotCol0 + (uint32_t)((set * kGroups + k) * kSlotCols);
                                 if constexpr (NS > 0) {  // a sum of its own for every block
-                                    const uint32_t db = tmem + (uint32_t)((set * kGroups + k) * NS);
+                                    const uint32_t db = tmem + (uint32_t)(((kSumSets == 2 ? set : 0) * kGroups + k) * NS);
 #pragma unroll
                                     for (int j = 0; j < 4; ++j) mma_ts(db, a + 8 * j, bd + 2 * j, p.idesc, j > 0);
                                 } else {
@@ -520,99 +539,117 @@ gemm_midrows_kernel(const __grid_constant__ CUtensorMap map_x, const MidParams p
         float4 e = e_next;
         int ch = 0;      // chunk
         int c_slot = 0;  // ring slot of the next item
-        // Block-scaled: the lane's row of the CTA's part of the tile, this group's blocks; the absmax of the
-        // blocks whose sums are still to come, of the chunk before (1) and the one before that (2)
-        float acc[NS > 0 ? NS : 1];
-        float am1 = 0.0f, am2 = 0.0f;
-        bool have1 = false, have2 = false;
-        auto add_block = [&](int set, float am) {
+        // Block-scaled: the lane's row of the CTA's part of the tile, the group's columns; how many blocks the
+        // chunk before has (1) and the one before that (2), where their sums are still to be added.
+        float acc[C];
+        int len1 = 0, len2 = 0;
+        // absmax of block k of chunk c, in the unused half of the table's lines: four chunks deep, a warp that
+        // writes chunk c has seen every warp through with chunk c - 4
+        auto am_at = [&](int c, int k) { return lut + (uint32_t)((((c & 3) * kGroups + k) * 4 + quarter) * 256 + 128 + lane * 4); };
+        auto add_blocks = [&](int c, int len) {  // absmax times block sum, blocks in order
+            ok = wait_spin(&done[c & 1], (c >> 1) & 1, p.limit, abort_flag) &&
+                 wait_spin(&a_full[c & 1], (c >> 1) & 1, p.limit, abort_flag);  // (over: orders the absmax values)
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) return;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t src = tmem + lane_off + (uint32_t)((kSumSets == 2 ? c & 1 : 0) * kGroups * NS + grp * C);
 #pragma unroll
-            for (int c0 = 0; c0 < NS; c0 += 16) {
-                float v[16];
-                tmem_ld16(tmem + lane_off + (uint32_t)((set * kGroups + grp) * NS + c0), v);
+            for (int k0 = 0; k0 < kGroups; k0 += 2) {
+                uint32_t v[2 * C];
+                tmem_ld_start(src + (uint32_t)(k0 * NS), v, std::integral_constant<int, C>{});
+                tmem_ld_start(src + (uint32_t)((k0 + 1) * NS), v + C, std::integral_constant<int, C>{});
+                float am[2];
 #pragma unroll
-                for (int i = 0; i < 16; ++i) acc[c0 + i] = fmaf(am, v[i], acc[c0 + i]);
+                for (int k = 0; k < 2; ++k) asm volatile("ld.shared.f32 %0, [%1];" : "=f"(am[k]) : "r"(am_at(c, k0 + k)));
+                tmem_landed(v);
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    if (k0 + k < len) {
+#pragma unroll
+                        for (int i = 0; i < C; ++i) acc[i] = fmaf(am[k], __uint_as_float(v[k * C + i]), acc[i]);
+                    }
+                }
             }
         };
-        // the warp's part of one chunk: block kb, or nothing (the chunk is short)
-        auto chunk = [&](int kb, bool have) {
+        auto give_up_decoding = [&]() {
+            if (lane == 0) give_up(kStatusTimeoutEmpty);
+        };
+        // the warp's part of one chunk of `len` blocks: block kb, or nothing (the chunk is short)
+        auto chunk = [&](int kb, bool have, int len) {
             const int set = ch & 1;
-            if (ch >= kSets) {  // the set's previous operands have been used
-                ok = wait_spin(&done[set], ((ch >> 1) - 1) & 1, p.limit, abort_flag);
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok) {
-                    if (lane == 0) give_up(kStatusTimeoutEmpty);
-                    return;
+            // the set's previous operands have been used; block-scaled: and their sums added, so that all of the
+            // set is free when this warp arrives
+            auto free_set = [&]() {
+                if (NS > 0 && kSumSets == 2) {
+                    if (len2 > 0) add_blocks(ch - 2, len2);
+                } else if (NS > 0) {  // one set of sums: those of the chunk before
+                    if (len1 > 0) add_blocks(ch - 1, len1);
+                } else if (ch >= kSets) {
+                    ok = wait_spin(&done[set], ((ch >> 1) - 1) & 1, p.limit, abort_flag);
+                    ok = __all_sync(0xffffffffu, ok);
                 }
-            }
-            ++ch;
-            if constexpr (NS > 0) {
-                if (have2) {  // (its set is this chunk's: both are free again when this warp arrives)
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    add_block(set, am2);
-                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                    __syncwarp();
-                }
-                have2 = have1;
-                am2 = am1;
-                have1 = have;
-            }
-            if (!have) {
-                if (lane == 0) mbar_arrive(&a_full[set]);
-                return;
-            }
-            asm volatile("cp.async.wait_group %0;" ::"n"(kDepth - 1) : "memory");
-            __syncwarp();  // (every lane's copies have landed)
-            const uint32_t src = ring + (uint32_t)(c_slot * kSlotBytes);
-            c_slot = c_slot == kDepth - 1 ? 0 : c_slot + 1;
-            const uint32_t mine = src + (uint32_t)(lane * 32), flip = (uint32_t)((row16 >> 2) & 1) * 16u;
-            const uint4 wa = lds_v4(mine + flip), wb = lds_v4(mine + (16u - flip));
-            float am;
-            if (p.kind == kAbsmaxCodes) {
-                uint32_t code;
-                asm volatile("ld.shared.u8 %0, [%1];" : "=r"(code) : "r"(src + 1024 + lane));
-                am = __fadd_rn(__fmul_rn(s_nmap[code], kb >= __float_as_int(e.z) ? e.y : e.x), e.w);
-            } else {
-                asm volatile("ld.shared.f32 %0, [%1];" : "=f"(am) : "r"(src + 1024 + 4 * lane));
-            }
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t dst = tmem + lane_off + kSlotCol0 + (uint32_t)((set * kGroups + grp) * kSlotCols);
-            // stored byte 8 t + 2 j + e covers k = 16 j + 4 t + 2 e: operand column 8 j + 2 t + e
-            const uint32_t ws[8] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
-            uint64_t am_pair;
-            asm("mov.b64 %0, {%1, %1};" : "=l"(am_pair) : "f"(am));
-            if constexpr (NS > 0) am1 = am;
-            auto pair = [&](auto byte, uint32_t word) {
-                if constexpr (NS > 0) return lookup2<decltype(byte)::value>(word, lut_lane);
-                else return decode2<decltype(byte)::value>(word, lut_lane, am_pair);
+                if (!ok) give_up_decoding();
+                return ok;
             };
-            using B0 = std::integral_constant<int, 0>;
-            using B1 = std::integral_constant<int, 1>;
-            using B2 = std::integral_constant<int, 2>;
-            using B3 = std::integral_constant<int, 3>;
-            uint32_t o[16];
+            if (kSumSets == 2 && !free_set()) return;
+            const uint32_t dst = tmem + lane_off + kSlotCol0 + (uint32_t)((set * kGroups + grp) * kSlotCols);
+            if (have) {
+                asm volatile("cp.async.wait_group %0;" ::"n"(kDepth - 1) : "memory");
+                __syncwarp();  // (every lane's copies have landed)
+                const uint32_t src = ring + (uint32_t)(c_slot * kSlotBytes);
+                c_slot = c_slot == kDepth - 1 ? 0 : c_slot + 1;
+                const uint32_t mine = src + (uint32_t)(lane * 32), flip = (uint32_t)((row16 >> 2) & 1) * 16u;
+                const uint4 wa = lds_v4(mine + flip), wb = lds_v4(mine + (16u - flip));
+                float am;
+                if (p.kind == kAbsmaxCodes) {
+                    uint32_t code;
+                    asm volatile("ld.shared.u8 %0, [%1];" : "=r"(code) : "r"(src + 1024 + lane));
+                    am = __fadd_rn(__fmul_rn(s_nmap[code], kb >= __float_as_int(e.z) ? e.y : e.x), e.w);
+                } else {
+                    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(am) : "r"(src + 1024 + 4 * lane));
+                }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                // stored byte 8 t + 2 j + e covers k = 16 j + 4 t + 2 e: operand column 8 j + 2 t + e
+                const uint32_t ws[8] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
+                uint64_t am_pair;
+                asm("mov.b64 %0, {%1, %1};" : "=l"(am_pair) : "f"(am));
+                if constexpr (NS > 0) asm volatile("st.shared.f32 [%0], %1;" ::"r"(am_at(ch, grp)), "f"(am) : "memory");
+                auto pair = [&](auto byte, uint32_t word) {
+                    if constexpr (NS > 0) return lookup2<decltype(byte)::value>(word, lut_lane);
+                    else return decode2<decltype(byte)::value>(word, lut_lane, am_pair);
+                };
+                using B0 = std::integral_constant<int, 0>;
+                using B1 = std::integral_constant<int, 1>;
+                using B2 = std::integral_constant<int, 2>;
+                using B3 = std::integral_constant<int, 3>;
+                uint32_t o[16];
 #pragma unroll
-            for (int t = 0; t < 4; ++t) {  // j = 0, 1: the low words of the 8-byte chunks
-                o[2 * t + 0] = pair(B0{}, ws[2 * t]);
-                o[2 * t + 1] = pair(B1{}, ws[2 * t]);
-                o[8 + 2 * t + 0] = pair(B2{}, ws[2 * t]);
-                o[8 + 2 * t + 1] = pair(B3{}, ws[2 * t]);
-            }
-            tmem_st16(dst, o);
-            uint32_t o2[16];
+                for (int t = 0; t < 4; ++t) {  // j = 0, 1: the low words of the 8-byte chunks
+                    o[2 * t + 0] = pair(B0{}, ws[2 * t]);
+                    o[2 * t + 1] = pair(B1{}, ws[2 * t]);
+                    o[8 + 2 * t + 0] = pair(B2{}, ws[2 * t]);
+                    o[8 + 2 * t + 1] = pair(B3{}, ws[2 * t]);
+                }
+                tmem_st16(dst, o);
+                uint32_t o2[16];
 #pragma unroll
-            for (int t = 0; t < 4; ++t) {  // j = 2, 3: the high words
-                o2[2 * t + 0] = pair(B0{}, ws[2 * t + 1]);
-                o2[2 * t + 1] = pair(B1{}, ws[2 * t + 1]);
-                o2[8 + 2 * t + 0] = pair(B2{}, ws[2 * t + 1]);
-                o2[8 + 2 * t + 1] = pair(B3{}, ws[2 * t + 1]);
+                for (int t = 0; t < 4; ++t) {  // j = 2, 3: the high words
+                    o2[2 * t + 0] = pair(B0{}, ws[2 * t + 1]);
+                    o2[2 * t + 1] = pair(B1{}, ws[2 * t + 1]);
+                    o2[8 + 2 * t + 0] = pair(B2{}, ws[2 * t + 1]);
+                    o2[8 + 2 * t + 1] = pair(B3{}, ws[2 * t + 1]);
+                }
+                tmem_st16(dst + 16, o2);
+                fetch();  // (every lane has used the slot's words: tcgen05.st is warp-wide)
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             }
-            tmem_st16(dst + 16, o2);
-            fetch();  // (every lane has used the slot's words: tcgen05.st is warp-wide)
-            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            if (kSumSets == 1 && !free_set()) return;
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) mbar_arrive(&a_full[set]);
+            ++ch;
+            len2 = kSumSets == 2 ? len1 : 0;
+            len1 = NS > 0 ? len : 0;
         };
 
         const int chunks = (p.M + 7) >> 3;    // accumulator columns in use, in eights
@@ -628,43 +665,20 @@ gemm_midrows_kernel(const __grid_constant__ CUtensorMap map_x, const MidParams p
             if (le < n) e_next = row_scale(tile + 1);
             if constexpr (NS > 0) {
 #pragma unroll
-                for (int i = 0; i < NS; ++i) acc[i] = 0.0f;
+                for (int i = 0; i < C; ++i) acc[i] = 0.0f;
             }
-            for (int j = grp; j < (le - ls + kGroups - 1) / kGroups * kGroups && ok; j += kGroups) chunk(kb0 + j, j < le - ls);
+            for (int j = 0; j < le - ls && ok; j += kGroups) chunk(kb0 + j + grp, j + grp < le - ls, min(kGroups, le - ls - j));
             if (!ok) break;
+            // ---- the tile's sums: the last blocks', or the accumulator ----
+            const int b = seg % bufs;
             if constexpr (NS > 0) {
-                // ---- the last blocks' sums; the group's row to tensor memory, where the groups meet ----
-#pragma unroll
-                for (int back = 2; back > 0; --back) {
-                    if ((back == 2 ? have2 : have1) && ok) {
-                        const int c0 = ch - back;
-                        ok = wait_spin(&done[c0 & 1], (c0 >> 1) & 1, p.limit, abort_flag);
-                        ok = __all_sync(0xffffffffu, ok);
-                        if (ok) {
-                            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                            add_block(c0 & 1, back == 2 ? am2 : am1);
-                        }
-                    }
-                }
-                have1 = have2 = false;
-                if (ok) {
-#pragma unroll
-                    for (int c0 = 0; c0 < NS; c0 += 16) {
-                        uint32_t r[16];
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) r[i] = __float_as_uint(acc[c0 + i]);
-                        tmem_st16(tmem + lane_off + (uint32_t)(grp * NS + c0), r);
-                    }
-                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&acc_full[0]);
-                }
+                if (len2 > 0) add_blocks(ch - 2, len2);
+                if (ok && len1 > 0) add_blocks(ch - 1, len1);
+                len1 = len2 = 0;
+            } else {
+                ok = wait_spin(&acc_full[b], (seg / bufs) & 1, p.limit, abort_flag);
+                ok = __all_sync(0xffffffffu, ok);
             }
-            // ---- drain the accumulator ----
-            const int b = NS > 0 ? 0 : seg % bufs;
-            if (ok) ok = wait_spin(&acc_full[b], (NS > 0 ? seg : seg / bufs) & 1, p.limit, abort_flag);
-            ok = __all_sync(0xffffffffu, ok);
             if (!ok) {
                 if (lane == 0) give_up(kStatusTimeoutTmem);
                 break;
@@ -676,39 +690,33 @@ gemm_midrows_kernel(const __grid_constant__ CUtensorMap map_x, const MidParams p
                 waited = true;
             }
             const uint32_t dcol = tmem + lane_off + (uint32_t)(b * 128);
-            auto sums8 = [&](int ch8, float (&v)[8]) {  // eight columns of the lane's row
-                tmem_ld8(dcol + (uint32_t)(ch8 * 8), v);
+            // this thread's columns of the row, C at a time
+            auto for_sums = [&](auto use) {
                 if constexpr (NS > 0) {
-#pragma unroll
-                    for (int g = 1; g < kGroups; ++g) {
-                        float w[8];
-                        tmem_ld8(dcol + (uint32_t)(g * NS + ch8 * 8), w);
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) v[i] += w[i];
+                    use(grp * C, acc);
+                } else {
+                    for (int ch = grp; ch < chunks; ch += kGroups) {
+                        float v[C];
+                        tmem_ld8(dcol + (uint32_t)(ch * 8), v);
+                        use(ch * 8, v);
+                        __syncwarp();  // (lanes past the output left early; the next load is warp-wide)
                     }
                 }
             };
             const bool whole = kb0 == 0 && le - ls == KB;
             const size_t part = (size_t)kTileM * p.NB;
             if (p.split <= 1 && whole) {
-                for (int ch = grp; ch < chunks; ch += kGroups) {
-                    float v[8];
-                    sums8(ch, v);
-                    emit(p, tile, quarter, lane, ch * 8, v);
-                    __syncwarp();  // (lanes past the output left early; the next load is warp-wide)
-                }
+                for_sums([&](int m0, float (&v)[C]) { emit(p, tile, quarter, lane, m0, v); });
             } else {
                 // partial tile, to shared memory (every copy, look-up and MMA of this CTA is through with
                 // it) or to the scratch
-                float4* o = p.split > 1 ? reinterpret_cast<float4*>(mid_smem + kPart)
+                float4* o = p.split > 1 ? reinterpret_cast<float4*>(mid_smem + (NS > 0 ? kPartScaled : kPart))
                                         : reinterpret_cast<float4*>(p.partials + ((size_t)c * 2 + (kb0 == 0 ? 1 : 0)) * part);
-                for (int ch = grp; ch < chunks; ch += kGroups) {
-                    float v[8];
-                    sums8(ch, v);
-                    float4* at = o + (size_t)ch * 2 * kTileM + row;
-                    at[0] = make_float4(v[0], v[1], v[2], v[3]);
-                    at[kTileM] = make_float4(v[4], v[5], v[6], v[7]);
-                }
+                for_sums([&](int m0, float (&v)[C]) {
+#pragma unroll
+                    for (int i = 0; i < C; i += 4)
+                        o[(size_t)(m0 + i) / 4 * kTileM + row] = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+                });
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
@@ -778,7 +786,7 @@ gemm_midrows_kernel(const __grid_constant__ CUtensorMap map_x, const MidParams p
         const int fours = warp >= kFirstDecodeWarp && !*abort_flag ? (p.M + 3) >> 2 : 0;
         bool arrived = false;
         for (int c4 = rank * kGroups + grp; c4 < fours; c4 += S * kGroups) {
-            float4* mine = reinterpret_cast<float4*>(mid_smem + kPart) + (size_t)c4 * kTileM + row;
+            float4* mine = reinterpret_cast<float4*>(mid_smem + (NS > 0 ? kPartScaled : kPart)) + (size_t)c4 * kTileM + row;
             float4 a[8];
 #pragma unroll
             for (int s = 0; s < 8; ++s) a[s] = s < S ? *cluster.map_shared_rank(mine, s) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -821,7 +829,7 @@ const MidDevice& mid_device(int dev) {
     static std::once_flag once[64];
     MidDevice& d = devs[dev];
     std::call_once(once[dev], [&] {
-        for (MidKernel k : {gemm_midrows_kernel<0>, gemm_midrows_kernel<16>, gemm_midrows_kernel<32>})
+        for (MidKernel k : {gemm_midrows_kernel<0>, gemm_midrows_kernel<16>, gemm_midrows_kernel<32>, gemm_midrows_kernel<48>})
             if (d.err == cudaSuccess)
                 d.err = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
         for (int s = 1; s <= 8 && d.err == cudaSuccess; ++s) {
@@ -972,8 +980,9 @@ AilaNf4Status launch_gemm_midrows(const AilaNf4Linear& w, AilaNf4Scratch& sc, co
         ++cfg.numAttrs;
     }
     const MidKernel kernel = !block_scaled ? gemm_midrows_kernel<0>
-                             : rows <= 16  ? gemm_midrows_kernel<16>
-                                           : gemm_midrows_kernel<32>;
+                             : p.NB == 16  ? gemm_midrows_kernel<16>
+                             : p.NB == 32  ? gemm_midrows_kernel<32>
+                                           : gemm_midrows_kernel<48>;
     const cudaError_t le = cudaLaunchKernelEx(&cfg, kernel, map_x, p);
     if (le != cudaSuccess) return cuda_fail(le, "gemm_midrows_kernel launch");
     return AILA_NF4_OK;

@@ -76,7 +76,7 @@ def test_linear(nf4, scratch, n, k, blocksize, nested, m):
     (6144, 2560, 64, True), (40000, 128, 128, False)])
 @pytest.mark.parametrize("m", [31, 32, 33, 47, 48, 49])
 def test_linear_at_the_edges_of_the_block_scaled_form(nf4, scratch, n, k, blocksize, nested, m):
-    """Its one pass of 32 rows, two passes, and the first row count of the other form."""
+    """Its widths of 32 and 48 rows, and the first row count of the other form."""
     test_linear(nf4, scratch, n, k, blocksize, nested, m)
 
 

@@ -86,8 +86,8 @@ def test_settings_choose_the_kernel(env, want):
 
 
 @pytest.mark.parametrize("n,k,rows,want", [
-    (18944, 256, (9, 49, 256), [MID] * 3), (18945, 256, (9, 49, 256), [SLICED, GEMM, GEMM]),
-    (18945, 448, (48,), [SLICED]), (18945, 512, (16, 17, 256, 257), [SLICED, MID, MID, GEMM]),
+    (18944, 256, (9, 49, 256), [MID] * 3), (18945, 256, (9, 17, 48, 49), [SLICED, MID, MID, GEMM]),
+    (18945, 192, (48,), [SLICED]), (18945, 448, (256,), [GEMM]), (18945, 512, (16, 17, 256, 257), [SLICED, MID, MID, GEMM]),
     (18945, 960, (16, 384), [SLICED, GEMM]), (18945, 1024, (9, 384), [MID, GEMM]),
     (512, 1472, (256, 257), [MID, GEMM]), (512, 1536, (256, 257), [MID, MID]), (65536, 1024, (384,), [MID])])
 def test_shapes_choose_the_kernel(n, k, rows, want):
