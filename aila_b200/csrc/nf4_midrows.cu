@@ -592,6 +592,11 @@ gemm_midrows_kernel(const __grid_constant__ CUtensorMap map_x, const MidParams p
                 return ok;
             };
             if (kSumSets == 2 && !free_set()) return;
+            if (NS == 0 && !have) {  // (nothing to publish)
+                ++ch;
+                if (lane == 0) mbar_arrive(&a_full[set]);
+                return;
+            }
             const uint32_t dst = tmem + lane_off + kSlotCol0 + (uint32_t)((set * kGroups + grp) * kSlotCols);
             if (have) {
                 asm volatile("cp.async.wait_group %0;" ::"n"(kDepth - 1) : "memory");
