@@ -4,6 +4,10 @@ the code-book value rounded to bf16 times the fp32 absmax, which is what the sma
 multiply by and closer to the unrounded weight. With the weights equal, what is left is the order of an fp32
 sum and the rounding of the result to bf16 (8 significant bits: at most 2^-8 of the value; twice more where
 gate and up pass through bf16)."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 import torch
@@ -225,3 +229,46 @@ def test_residual_of_the_launch_before(nf4, m):
                 torch.cuda.synchronize()
         assert torch.equal(t, x), rep
     sc.check()
+
+
+@pytest.mark.parametrize("m", [9, 40, 77, 256, 384])
+def test_linear_it_does_not_take(nf4, scratch, m):
+    """More than 256 absmax codes per row: no table of row scales, so batched decode launches up to 48 rows and
+    the dequantise + GEMM route above serve these row counts (sums of the former in no fixed order)."""
+    n, k = 200, 25600
+    lin = _linear(nf4, 61, n, k)
+    w = _weight(lin, [make_weight(61, n, k)], m)
+    x, res = _x(m, m, k), _x(m + 1, m, n)
+    y = torch.full((m + 1, n), 7.0, dtype=torch.bfloat16, device="cuda")
+    lin.forward(scratch, x, y[:m], m, res)
+    want = x.double() @ w + res.double()
+    assert ((y[:m].double() - want).abs() <= 2 ** -8 * want.abs() + 1e-5 * (x.double().abs() @ w.abs())).all()
+    assert (y[m] == 7.0).all()
+    scratch.check()
+
+
+SPLITS = r"""
+import torch
+from aila_b200 import linear as nf4
+from tests import test_midrows_gpu as t
+sc = nf4.Bnb4BitLinearScratch(0)
+# K of 1, 5, 7, 16 and 65 blocks: shares of a cluster's CTAs that are equal, unequal and short of a chunk
+for n, k, bs, nested in ((200, 64, 64, True), (129, 320, 64, False), (100, 448, 64, True), (300, 1024, 128, True),
+                         (1000, 4160, 64, False)):
+    for m in (9, 17, 48, 49, 129, 256):
+        t.test_linear(nf4, sc, n, k, bs, nested, m)
+for ff, k in ((80, 448), (1040, 512)):
+    for m in (9, 40, 77, 200):
+        t.test_gate_up(nf4, sc, ff, k, m)
+print("splits ok")
+"""
+
+
+@pytest.mark.parametrize("split", range(9))
+def test_every_split(split):
+    """The stream split and clusters of one to eight CTAs, each forced on small ragged shapes (the choice is read
+    once per process)."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    env = dict(os.environ, AILA_NF4_MID_SPLIT=str(split), PYTHONPATH=root)
+    r = subprocess.run([sys.executable, "-c", SPLITS], cwd=root, env=env, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "splits ok" in r.stdout, r.stdout[-1000:] + r.stderr[-3000:]

@@ -609,9 +609,8 @@ def test_argmax_bf16(nf4):
 
 @pytest.mark.parametrize("M", [2, 5, 8, 9, 17, 32, 33, 41, 48, 49, 65])
 def test_small_batch_routes_agree(nf4, oracle, scratch, M):
-    """2..48 rows take the small-batch decode kernels (launches of up to 32 rows, one weight pass
-    each), more rows the dequantise + GEMM route: both must meet the bound against the oracle's
-    forward."""
+    """Few rows take a batched decode kernel or the tensor-memory kernel, or the dequantise + GEMM route where
+    the settings say so: all must meet the bound against the oracle's forward."""
     N, K = 272, 512
     w = make_weight(8100 + M, N, K)
     lin = _lin(nf4, w)

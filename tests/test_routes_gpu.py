@@ -114,3 +114,13 @@ def test_shapes_choose_the_kernel(n, k, rows, want):
     assert got == want
     lin.close()
     sc.close()
+
+
+def test_gemm_route_at_fewer_rows():
+    """The prefill tests at 49 to 384 rows once more with the tensor-memory kernel switched off: the dequantisation
+    pass and the GEMM's 128-row tiles, which serve linears that the kernel does not take."""
+    r = subprocess.run([sys.executable, "-m", "pytest", "tests/test_parity_gpu.py", "-q", "-m", "gpu", "-p", "no:cacheprovider",
+                        "-k", "prefill or small_batch_routes_agree"], cwd=ROOT,
+                       env=dict(os.environ, AILA_NF4_MID_ROWS_MAX="0", PYTHONPATH=ROOT), capture_output=True, text=True,
+                       timeout=600)
+    assert r.returncode == 0 and " passed" in r.stdout, r.stdout[-3000:] + r.stderr[-1000:]
