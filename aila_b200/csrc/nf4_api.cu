@@ -325,7 +325,8 @@ AilaNf4Status ensure_weight(AilaNf4Scratch* sc, size_t bytes) {
     NF4_CUDA(e);
     sc->weight_bytes = bytes;
     // whoever may run the GEMM route under capture may run the tensor-memory kernel with fewer rows
-    return nf4::ensure_mid_partials(sc);
+    nf4::try_mid_partials(sc);
+    return AILA_NF4_OK;
 }
 
 using nf4::ensure_counters;
@@ -481,11 +482,11 @@ AilaNf4Status run_mid_rows(const AilaNf4Linear* l, AilaNf4Scratch* sc, const voi
     AilaNf4Status st = ensure_counters(sc, (size_t)nf4::gemm_midrows_tiles(*l, ff_dim));
     if (st != AILA_NF4_OK) return st;
     // The first call that is not captured allocates the partial tiles whatever split it takes itself: after
-    // it, calls of every split can be captured. (A captured first call fails only where its split needs them.)
+    // it, calls of every split can be captured.
     if (!sc->d_mid_partials) {
         cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
         NF4_CUDA(cudaStreamIsCapturing(s, &capture));
-        if (capture == cudaStreamCaptureStatusNone && (st = nf4::ensure_mid_partials(sc)) != AILA_NF4_OK) return st;
+        if (capture == cudaStreamCaptureStatusNone) nf4::try_mid_partials(sc);
     }
     // Up to 48 rows, where the small-batch decode kernels serve otherwise, the code-book value alone is rounded to
     // bf16, as there; above, the weight, as on the dequantise + GEMM route.
@@ -557,11 +558,14 @@ namespace nf4 {
 
 // Partial tiles of the tensor-memory kernel's stream split, one size for every call (39 MB on 148 SMs):
 // captured launches keep the address, so the buffer neither grows nor moves until the scratch is destroyed.
-AilaNf4Status ensure_mid_partials(AilaNf4Scratch* sc) {
-    if (sc->d_mid_partials) return AILA_NF4_OK;
-    NF4_CUDA(cudaMalloc(reinterpret_cast<void**>(&sc->d_mid_partials),
-                        gemm_midrows_partial_bytes(sc->sm_count, kMidRowsMax)));
-    return AILA_NF4_OK;
+// Without it (no memory left, or a first call under capture) the kernel takes clusters.
+void try_mid_partials(AilaNf4Scratch* sc) {
+    if (sc->d_mid_partials) return;
+    if (cudaMalloc(reinterpret_cast<void**>(&sc->d_mid_partials),
+                   gemm_midrows_partial_bytes(sc->sm_count, kMidRowsMax)) != cudaSuccess) {
+        sc->d_mid_partials = nullptr;
+        cudaGetLastError();
+    }
 }
 
 AilaNf4Status ensure_counters(AilaNf4Scratch* sc, size_t tiles) {
@@ -860,8 +864,7 @@ AILA_NF4_API AilaNf4Status aila_nf4_scratch_reserve(AilaNf4Scratch* sc, int seq_
         st = ensure_rows_acc(sc, tiles * nf4::kTileRows * 32 * sizeof(float));
         if (st != AILA_NF4_OK) return st;
         // partial tiles of the tensor-memory kernel (calls that are captured allocate nothing)
-        st = nf4::ensure_mid_partials(sc);
-        if (st != AILA_NF4_OK) return st;
+        nf4::try_mid_partials(sc);
     }
     if (need_weight) {
         st = ensure_weight(sc, (size_t)in_features * (size_t)out_features * 2);

@@ -199,7 +199,7 @@ constexpr int kMidRowsScaled = 48;  // of the block-scaled form: operand bf16(co
 bool gemm_midrows_supported(const AilaNf4Linear& w, int64_t swiglu_ff);
 int gemm_midrows_tiles(const AilaNf4Linear& w, int64_t swiglu_ff);  // counters it needs
 size_t gemm_midrows_partial_bytes(int ctas, int rows);  // of the stream split
-AilaNf4Status ensure_mid_partials(AilaNf4Scratch* sc);
+void try_mid_partials(AilaNf4Scratch* sc);
 AilaNf4Status launch_gemm_midrows(const AilaNf4Linear& w, AilaNf4Scratch& sc, const void* x, void* y,
                                   const void* residual, int rows, int64_t swiglu_ff, bool block_scaled, cudaStream_t s);
 

@@ -869,23 +869,23 @@ constexpr SplitCost kCostScaled = {0.66, 0.68, 2.08, 1.40, 2.97, 2.77, 1.63, 1.7
 constexpr SplitCost kCostPlain = {0.78, 0.21, 1.29, 1.66, 2.51, 1.84, 1.83, 2.17,
                                   1.00, 0.57, 0.68, 0.53, 0.00, 0.57, 0.52, 2.50, 5.48};
 
-// 0: the stream split; else CTAs per tile. On the measured shapes the choice is 0.4 % behind the best split on
+// 0: the stream split (where there are partial tiles for it); else CTAs per tile. On the measured shapes the choice is 0.4 % behind the best split on
 // average and 10 % at worst (10 % on average and 57 % at worst by the model of one layer's width before it:
 // 6144x2560 at 32 rows 14.9 -> 9.5 us, 30000x512 at 256 rows 30.2 -> 20.4 us).
-int choose_split(const MidDevice& d, int n_tiles, int KB, int NB, bool block_scaled, int sm_count) {
+int choose_split(const MidDevice& d, int n_tiles, int KB, int NB, bool block_scaled, bool stream, int sm_count) {
     static const int forced = [] {  // for measurements: AILA_NF4_MID_SPLIT=0..8
         const char* e = std::getenv("AILA_NF4_MID_SPLIT");
         return e && *e ? std::atoi(e) : -1;
     }();
-    if (forced >= 0 && forced <= 8 && forced <= KB) return forced;
+    if (forced >= (stream ? 0 : 1) && forced <= 8 && forced <= KB) return forced;
     const SplitCost& c = block_scaled ? kCostScaled : kCostPlain;
     const double cols = NB / 100.0;
     const int64_t total = (int64_t)n_tiles * KB;
     const int64_t ctas = (total + 7) / 8 < sm_count ? (total + 7) / 8 : sm_count;
     const double items = (double)total / ctas, tiles = items / KB;
     double best = 1e30;
-    int split = 0;
-    if (ctas <= 8 * (int64_t)n_tiles)  // (a tile's last CTA adds all parts: not more than a cluster has)
+    int split = stream ? 0 : 1;
+    if (stream && ctas <= 8 * (int64_t)n_tiles)  // (a tile's last CTA adds all parts: not more than a cluster has)
         best = items / 4 * (c.s_chunk + c.s_chunk_col * cols) + tiles * (c.tile + c.tile_col * cols) +
                (1 / tiles > 2 ? (1 / tiles - 2) * (c.join + c.join_col * cols) : 0) + c.launch + c.launch_col * cols +
                (2 * ctas > sm_count ? c.s_alone : 0);
@@ -958,15 +958,11 @@ AilaNf4Status launch_gemm_midrows(const AilaNf4Linear& w, AilaNf4Scratch& sc, co
     cudaGetDevice(&dev);
     const MidDevice& md = mid_device(dev & 63);
     if (md.err != cudaSuccess) return cuda_fail(md.err, "cudaFuncSetAttribute(gemm_midrows)");
-    p.split = choose_split(md, p.n_tiles, p.KU, p.NB, block_scaled, sc.sm_count);
+    p.split = choose_split(md, p.n_tiles, p.KU, p.NB, block_scaled, sc.d_mid_partials != nullptr, sc.sm_count);
     const int64_t total = (int64_t)p.n_tiles * p.KU;
     const int64_t want = p.split > 0 ? (int64_t)p.n_tiles * p.split : (total + 7) / 8;  // stream: eight items per CTA at least
     const int grid = (int)(p.split > 0 || want < sc.sm_count ? want : sc.sm_count);
-    if (p.split == 0) {
-        const AilaNf4Status st = ensure_mid_partials(&sc);
-        if (st != AILA_NF4_OK) return st;
-        p.partials = sc.d_mid_partials;
-    }
+    p.partials = sc.d_mid_partials;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
     cfg.blockDim = dim3(kThreads);

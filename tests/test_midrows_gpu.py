@@ -196,6 +196,28 @@ def test_capture_after(nf4, before):
     sc.check()
 
 
+@pytest.mark.parametrize("m", [32, 77])
+def test_captured_first_call(nf4, m):
+    """Nothing can be allocated in a captured first call: the tiles that would be cut over the whole chip go to
+    clusters."""
+    n, k = 19456, 2560
+    lin = _linear(nf4, 9, n, k)
+    w = _weight(lin, [make_weight(9, n, k)], m)
+    sc = nf4.Bnb4BitLinearScratch(0)
+    x, y = _x(m, m, k), torch.zeros(m, n, dtype=torch.bfloat16, device="cuda")
+    torch.cuda.synchronize()
+    st = torch.cuda.Stream()
+    with torch.cuda.stream(st):
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=st):
+            lin.forward(sc, x, y, m)
+        graph.replay()
+    torch.cuda.synchronize()
+    want = x.double() @ w
+    assert ((y.double() - want).abs() <= 2 ** -8 * want.abs() + 1e-5 * (x.double().abs() @ w.abs())).all()
+    sc.check()
+
+
 @pytest.mark.parametrize("m", [16, 77])
 def test_residual_of_the_launch_before(nf4, m):
     """The residual is what the launch before has just written, at the same address on every replay: it must
