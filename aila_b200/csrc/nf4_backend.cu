@@ -348,7 +348,7 @@ attention_cluster_kernel(const uint16_t* q, const uint16_t* k_cache, const uint1
 }
 
 constexpr size_t kAttMaxSmem = 220 * 1024;
-constexpr unsigned kAttFill = 132;  // CTAs that run at once, clusters of eight included
+constexpr size_t kAttTwoSmem = 112 * 1024;  // two CTAs on an SM (228 KB, 1 KB and the static arrays of each among them)
 
 struct AttentionPlan {
     void (*fn)(const uint16_t*, const uint16_t*, const uint16_t*, uint16_t*, int, int, const int*, int) = nullptr;
@@ -357,33 +357,65 @@ struct AttentionPlan {
     cudaError_t err = cudaSuccess;
 };
 
+// What the launches of one instantiation on one device need to know, found out once.
+struct AttentionDevice {
+    cudaError_t err = cudaSuccess;
+    int fit[2][9] = {};  // clusters of 1, 2, 4 or 8 CTAs that run at once, one or two CTAs on an SM
+};
+
+template <int HD, int HG>
+const AttentionDevice& attention_device(int device) {
+    static std::once_flag once[64];
+    static AttentionDevice devs[64];
+    AttentionDevice& d = devs[device & 63];
+    std::call_once(once[device & 63], [&] {
+        d.err = cudaFuncSetAttribute(attention_cluster_kernel<HD, HG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)kAttMaxSmem);
+        for (int two = 0; two < 2; ++two) {
+            for (unsigned ctas = 1; ctas <= 8 && d.err == cudaSuccess; ctas *= 2) {
+                cudaLaunchConfig_t cfg = {};
+                cfg.gridDim = dim3(ctas * 1024);
+                cfg.blockDim = dim3(kAttThreads);
+                cfg.dynamicSmemBytes = two ? kAttTwoSmem : kAttMaxSmem;
+                cudaLaunchAttribute attr[1];
+                attr[0].id = cudaLaunchAttributeClusterDimension;
+                attr[0].val.clusterDim.x = ctas;
+                attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+                cfg.attrs = attr;
+                cfg.numAttrs = 1;
+                d.err = cudaOccupancyMaxActiveClusters(&d.fit[two][ctas], attention_cluster_kernel<HD, HG>, &cfg);
+            }
+        }
+    });
+    return d;
+}
+
+// Takes the group size if it divides the heads and holds the scores; whether all of its clusters run at once.
 template <int HD, int HG>
 bool attention_plan(int heads, int per_kv, int cached_len, unsigned ctas, int device, AttentionPlan* plan) {
     const size_t smem = attention_cluster_smem<HD, HG>(cached_len);
     if (per_kv % HG != 0 || smem > kAttMaxSmem) return false;
-    if (HG > 1 && (unsigned)(heads / HG) * ctas * 2 <= kAttFill) return false;
+    const AttentionDevice& d = attention_device<HD, HG>(device);
     plan->fn = attention_cluster_kernel<HD, HG>;
     plan->smem = smem;
     plan->hg = HG;
-    static std::once_flag once[64];
-    static cudaError_t err[64];
-    std::call_once(once[device & 63], [&] {
-        err[device & 63] = cudaFuncSetAttribute(attention_cluster_kernel<HD, HG>,
-                                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAttMaxSmem);
-    });
-    plan->err = err[device & 63];
-    return true;
+    plan->err = d.err;
+    return heads / HG <= d.fit[smem <= kAttTwoSmem ? 1 : 0][ctas];
 }
 
-// Head groups of four, two or one share what they read: as large as the scores of the window leave room for,
-// but halved while twice the CTAs still run at once (each holds more than 100 KB of shared memory, one per
-// SM): a CTA's work is a chain of latencies. 32 heads over 1001 positions take 20.0 us in groups of four, 18.4 us
-// in groups of two (cold L2).
+// Head groups of four, two or one share what they read, but a CTA's work is a chain of latencies: the smallest
+// group whose clusters all run at once, and where none does the largest that holds its scores. us per launch by
+// group size (24 caches in turn, best of the rule in brackets):
+//   32 heads of 128 on 8 key/value heads, 1000 positions: 18.9, 16.7, 13.8 in groups of four, two, one (one);
+//   4000 positions, where 15 clusters of eight run at once: 58.8, 98.7, 118 (four); 64 heads, 1000 positions:
+//   36.6, 18.3 in groups of four and two (two)
 template <int HD>
 bool attention_plan_of(int heads, int per_kv, int cached_len, unsigned ctas, int device, AttentionPlan* plan) {
-    return attention_plan<HD, 4>(heads, per_kv, cached_len, ctas, device, plan) ||
-           attention_plan<HD, 2>(heads, per_kv, cached_len, ctas, device, plan) ||
-           attention_plan<HD, 1>(heads, per_kv, cached_len, ctas, device, plan);
+    plan->fn = nullptr;
+    if (!attention_plan<HD, 1>(heads, per_kv, cached_len, ctas, device, plan) &&
+        !attention_plan<HD, 2>(heads, per_kv, cached_len, ctas, device, plan))
+        attention_plan<HD, 4>(heads, per_kv, cached_len, ctas, device, plan);
+    return plan->fn != nullptr;
 }
 
 struct BackendDevGuard {

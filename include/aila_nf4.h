@@ -137,8 +137,9 @@ AILA_NF4_API void aila_nf4_scratch_destroy(AilaNf4Scratch* scratch);
  * Pre-size the work space so later forward calls never allocate (call before capturing a
  * CUDA graph). Mirrors Bnb4BitLinearScratch::ensure (src/ops/Bnb4BitLinear.cpp:414-451);
  * need_weight != 0 reserves the [out,in] bf16 weight buffer the seq_len > 1 route uses; seq_len > 1
- * also reserves the fp32 accumulation tiles of the small-batch decode kernel (128 bytes per output row)
- * and the partial tiles of the tensor-memory kernel (256 KB per SM, allocated once and never moved).
+ * also reserves the fp32 accumulation tiles of the small-batch decode kernel (128 bytes per output row).
+ * Both reserve the partial tiles of the tensor-memory kernel (256 KB per SM, allocated once and never moved;
+ * without them, for want of memory, the kernel cuts its work so that it needs none).
  * A decode call for more than 262,144 output rows that was not reserved for grows the work space
  * inside the call: it allocates and waits for the device, so it cannot be captured.
  */
@@ -158,11 +159,13 @@ AILA_NF4_API AilaNf4Status aila_nf4_scratch_check(AilaNf4Scratch* scratch, void*
  *   seq_len 2..8  -> one batched decode launch (one pass over the packed weights, fp32
  *                    accumulation; no reference counterpart: the reference takes its
  *                    seq_len > 1 route from two rows on);
- *   seq_len 9..384 -> weights rounded to bf16 exactly as dequantize_weight (:723-757) does,
- *                    decoded into the tensor-memory operand of a tcgen05 kernel, up to 256 rows
- *                    per pass over the packed weights; linears without a per-row scale table
- *                    (8-bit absmax codes and more than 256 absmax blocks per row) take batched
- *                    decode launches up to 48 rows;
+ *   seq_len 9..384 -> NF4 decoded into the tensor-memory operand of a tcgen05 kernel, up to 256
+ *                    rows per pass over the packed weights. Up to 48 rows the operand is the
+ *                    code-book value rounded to bf16, as in the batched decode launches, and the
+ *                    absmax stays an fp32 factor; above, the weight rounded to bf16 exactly as
+ *                    dequantize_weight (:723-757) does. Linears without a per-row scale table
+ *                    (8-bit absmax codes and more than 256 absmax blocks per row) and some with a
+ *                    short K take batched decode launches up to 48 rows and the next route above;
  *   above         -> weights rounded to bf16 exactly as dequantize_weight (:723-757) does,
  *                    then a tcgen05 tensor-core GEMM with fp32 accumulation (the reference
  *                    runs an oneDNN bf16 matmul, :689-721, :944). With blocksize 128 the

@@ -116,6 +116,14 @@ def test_attention_decode_cluster(be, heads, kv, hd, length):
     assert torch.allclose(out.cpu().double().view(heads, hd), want, rtol=2 ** -8, atol=1e-4)
 
 
+@pytest.mark.parametrize("heads,kv,hd,length", [
+    (32, 8, 128, 1000), (32, 8, 128, 4000), (64, 8, 128, 1000), (64, 8, 128, 4000), (48, 8, 64, 2000), (40, 8, 128, 300)])
+def test_attention_decode_head_groups(be, heads, kv, hd, length):
+    """Groups of one, two and four heads by what runs at once, more clusters than run at once, heads per key/value
+    head that only pairs or single heads divide."""
+    test_attention_decode_cluster(be, heads, kv, hd, length)
+
+
 def test_step_replayed_with_new_inputs(be):
     """q, k, v and the position are written by the launches right before and sit at the same addresses on
     every replay; the kernels that read them start before those launches end. 200 replayed steps against the
